@@ -360,13 +360,14 @@ int sb_encoder_backward(sb_encoder* enc, void* stream, const void* dy, void* con
  * CUDA events when timing was switched on; writes up to max (name, ms) pairs
  * and returns the count.  While timing is on every operator is also an NVTX range
  * of the same name on the calling thread (the ranges of pytorch_module/encoder.cu:32-53),
- * and passes are launched plainly rather than replayed as graphs. */
+ * and passes are launched plainly rather than as graphs. */
 int sb_encoder_set_timing(sb_encoder* enc, int enabled);
 int sb_encoder_get_timing(sb_encoder* enc, int max, const char** names, float* ms);
 /* Number of operators the most recent forward / backward launched. */
-/* A pass whose pointer arguments repeat (explicit masks, timing off) is captured once as a CUDA graph and
- * replayed with a single launch afterwards; 0 switches that off for the handle (default on; the environment
- * variable SUBSTATION_B200_GRAPHS=0 switches it off for the process). */
+/* From its second pass in a direction on, a handle runs passes as CUDA graphs whose kernel parameters are rewritten
+ * for every pass (any buffers, mask mode or offset; timing off): one graph launch instead of one launch per kernel.
+ * 0 switches that off for the handle (default on; the environment variable SUBSTATION_B200_GRAPHS=0 switches it off
+ * for the process). */
 int sb_encoder_set_graphs(sb_encoder* enc, int enabled);
 /* A CUDA event (cudaEvent_t, caller-owned; NULL to stop) that every backward pass records on its stream as soon
  * as the gradients of the feed-forward half and of both LayerNorms are final (LINW1, LINB1, LINW2, LINB2, S1,
@@ -374,7 +375,7 @@ int sb_encoder_set_graphs(sb_encoder* enc, int enabled);
  * the attention half of the backward pass runs.  A data-parallel host waits for it on its communication
  * stream and starts the allreduce of that part of the gradient bucket while the pass continues. */
 int sb_encoder_set_ffn_grads_event(sb_encoder* enc, void* event);
-/* How many passes were captured as graphs and how many were replayed since the handle was created. */
+/* How many passes were captured as graphs and how many ran as one since the handle was created. */
 int sb_encoder_graph_stats(sb_encoder* enc, long long* captures, long long* replays);
 int sb_encoder_launch_count(sb_encoder* enc);
 /* Kernels launched by the most recent forward plus the most recent backward (an operator may need

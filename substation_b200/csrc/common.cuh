@@ -10,6 +10,7 @@
 
 #include <cstring>
 #include <string>
+#include <tuple>
 
 #include "../../include/substation_b200.h"
 
@@ -177,6 +178,13 @@ inline int cached_blocks_per_sm(const void* kernel, int threads) {
 // Kernels launched through launch_k by this thread (the layer handle reports the difference over a pass).
 extern thread_local long long g_kernel_launches;
 
+// Where a thread's launches go instead of straight onto a stream: the layer handle records a pass into a CUDA graph
+// and, on later passes, rewrites the parameters of the recorded kernels (api.cu, run_pass).
+struct LaunchSink {
+  virtual cudaError_t put(const cudaLaunchConfig_t& cfg, const void* kernel, void** args) = 0;
+};
+extern thread_local LaunchSink* g_launch_sink;
+
 template <class... KArgs, class... Args>
 cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                      Args&&... args) {
@@ -192,7 +200,14 @@ cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t sme
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 1 : 0;
   ++g_kernel_launches;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+  std::tuple<KArgs...> values(static_cast<KArgs>(args)...);
+  return std::apply(
+      [&](auto&... v) {
+        void* ptrs[] = {const_cast<void*>(static_cast<const void*>(&v))...};
+        const void* fn = reinterpret_cast<const void*>(kernel);
+        return g_launch_sink ? g_launch_sink->put(cfg, fn, ptrs) : cudaLaunchKernelExC(&cfg, fn, ptrs);
+      },
+      values);
 }
 
 #define SB_LAUNCH_OK(expr)                                                              \

@@ -21,7 +21,6 @@ There is no CPU path: tensors must be on a CUDA device.
 """
 
 import ctypes
-import os
 import math
 
 import torch
@@ -36,15 +35,98 @@ def _round_up(n, a=_ALIGN):
     return (n + a - 1) // a * a
 
 
-# Replay of repeated passes as CUDA graphs inside the autograd path: off unless asked for.  The arenas, outputs
-# and gradients of that path come from torch's caching allocator, whose blocks do not repeat reliably from step
-# to step (measured: one capture per three steps, no gain), unlike the caller-held arenas of the raw passes.
-_AUTOGRAD_GRAPHS = os.environ.get('SUBSTATION_B200_AUTOGRAD_GRAPHS', '0') == '1'
-
 def _to_numpy(t):
     """numpy copy of a tensor for ``.debug``; numpy has no bfloat16, those come back as float32 (exact)."""
     t = t.detach()
     return (t.float() if t.dtype == torch.bfloat16 else t).cpu().numpy()
+
+
+class _EncoderFunction(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, outer, X, anchor, *weights):
+        ctx.outer = outer
+        # Hot path: one arena per pass, pointers computed from the plan's offsets; tensor views
+        # over the arena are only built when somebody asks for them (debug, or a caller of views()).
+        # ``anchor`` is None on the ordinary path (``weights`` are the sixteen parameters, and autograd routes
+        # their gradients).  With a buffer pool it is a one-element leaf that keeps the node in the graph,
+        # ``weights`` is ONE tuple of detached parameters that autograd does not look into, and backward
+        # writes every ``.grad`` itself: sixteen inputs and sixteen accumulation nodes less per step.
+        ctx.direct = anchor is not None
+        if ctx.direct:
+            weights = weights[0]
+        outer._check_input(X, 'X')
+        X = X.contiguous()
+        weights = tuple(w if w.is_contiguous() else w.contiguous() for w in weights)
+        plan, total = outer._fwd_plan
+        pooled = outer._pool_set(X) if outer.__dict__.get('_pool_n') else None
+        if pooled is not None:
+            Y, arena = pooled['Y'], pooled['fwd']
+            ctx.pool_set = pooled
+        else:
+            Y = torch.empty_like(X)
+            arena = torch.empty(max(total, 1), dtype=torch.uint8, device=X.device)
+            ctx.pool_set = None
+        over = outer._explicit_masks(X.device) if outer.mask_mode == 'explicit' else {}
+        ptrs = outer._pooled_ptrs('fwd', plan, arena, over) if pooled is not None else \
+            outer._plan_ptrs(plan, arena, over)
+        outer._forward_ptrs(X, weights, ptrs, Y)
+        if ctx.direct:
+            ctx.weights = weights
+            ctx.save_for_backward(arena, X)
+        else:
+            ctx.save_for_backward(*weights, arena, X)
+        ctx.masks = over
+        if outer.enable_debug:
+            torch.cuda.synchronize()
+            fwd = outer.views('forward', arena)
+            fwd.update(over)
+            for name in outer._fwd_names:
+                outer.debug[name] = _to_numpy(fwd[name])
+            for name, w in zip(outer._param_names, weights):
+                outer.debug[name] = _to_numpy(w)
+        return Y
+
+    @staticmethod
+    def backward(ctx, DY):
+        outer = ctx.outer
+        saved = ctx.saved_tensors
+        np_ = len(outer._param_names)
+        if ctx.direct:
+            weights, arena, X = ctx.weights, saved[0], saved[1]
+        else:
+            weights, arena, X = saved[:np_], saved[np_], saved[-1]
+        outer._check_input(DY, 'DY')
+        DY = DY.contiguous()
+        bplan, btotal = outer._bwd_plan
+        gplan, gtotal = outer._grad_plan
+        if ctx.pool_set is not None:
+            DX, barena = ctx.pool_set['DX'], ctx.pool_set['bwd']
+            garena = ctx.pool_set['grads'] if not outer.__dict__.get('_grad_arenas') else \
+                outer._next_grad_arena(gtotal, DY.device)
+        else:
+            DX = torch.empty_like(DY)
+            barena = torch.empty(max(btotal, 1), dtype=torch.uint8, device=DY.device)
+            garena = outer._next_grad_arena(gtotal, DY.device)
+        tab = outer._pooled_ptrs if ctx.pool_set is not None else \
+            (lambda which, plan, a, over: outer._plan_ptrs(plan, a, over))
+        outer._backward_ptrs(DY, tab('grads', gplan, garena, {}), tab('bwd', bplan, barena, {}), weights,
+                             tab('fwd', outer._fwd_plan[0], arena, ctx.masks), X, DX)
+        g16 = garena[:max(gtotal, 2)].view(outer.torch_dtype)
+        outer._grad_bucket = g16
+        grads = tuple(torch.as_strided(g16, shape, strides, off) for shape, strides, off in outer._grad_views)
+        if outer.enable_debug:
+            torch.cuda.synchronize()
+            bwd = outer.views('backward', barena)
+            for name in outer._bwd_names:
+                outer.debug[name] = _to_numpy(bwd[name])
+            for name, g in zip(outer._param_names, grads):
+                outer.debug['D' + name] = _to_numpy(g)
+        if ctx.direct:
+            for prm, g in zip(outer.params, grads):
+                if prm.requires_grad:
+                    prm.grad = g
+            return None, DX, None, None
+        return (None, DX, None, *grads)
 
 
 class Encoder(torch.nn.Module):
@@ -121,95 +203,6 @@ class Encoder(torch.nn.Module):
                 strides.append(acc)
                 acc *= extent
             self._grad_views.append((tuple(shape), tuple(reversed(strides)), off // 2))
-
-        outer = self
-
-        class EncoderFunction(torch.autograd.Function):
-            @staticmethod
-            def forward(ctx, X, anchor, *weights):
-                # Hot path: one arena per pass, pointers computed from the plan's offsets; tensor views
-                # over the arena are only built when somebody asks for them (debug, or a caller of views()).
-                # ``anchor`` is None on the ordinary path (``weights`` are the sixteen parameters, and autograd routes
-                # their gradients).  With a buffer pool it is a one-element leaf that keeps the node in the graph,
-                # ``weights`` is ONE tuple of detached parameters that autograd does not look into, and backward
-                # writes every ``.grad`` itself: sixteen inputs and sixteen accumulation nodes less per step.
-                ctx.direct = anchor is not None
-                if ctx.direct:
-                    weights = weights[0]
-                outer._check_input(X, 'X')
-                X = X.contiguous()
-                weights = tuple(w if w.is_contiguous() else w.contiguous() for w in weights)
-                plan, total = outer._fwd_plan
-                pooled = outer._pool_set(X) if outer.__dict__.get('_pool_n') else None
-                if pooled is not None:
-                    Y, arena = pooled['Y'], pooled['fwd']
-                    ctx.pool_set = pooled
-                else:
-                    Y = torch.empty_like(X)
-                    arena = torch.empty(max(total, 1), dtype=torch.uint8, device=X.device)
-                    ctx.pool_set = None
-                over = outer._explicit_masks(X.device) if outer.mask_mode == 'explicit' else {}
-                ptrs = outer._pooled_ptrs('fwd', plan, arena, over) if pooled is not None else \
-                    outer._plan_ptrs(plan, arena, over)
-                outer._forward_ptrs(X, weights, ptrs, Y)
-                if ctx.direct:
-                    ctx.weights = weights
-                    ctx.save_for_backward(arena, X)
-                else:
-                    ctx.save_for_backward(*weights, arena, X)
-                ctx.masks = over
-                if outer.enable_debug:
-                    torch.cuda.synchronize()
-                    fwd = outer.views('forward', arena)
-                    fwd.update(over)
-                    for name in outer._fwd_names:
-                        outer.debug[name] = _to_numpy(fwd[name])
-                    for name, w in zip(outer._param_names, weights):
-                        outer.debug[name] = _to_numpy(w)
-                return Y
-
-            @staticmethod
-            def backward(ctx, DY):
-                saved = ctx.saved_tensors
-                np_ = len(outer._param_names)
-                if ctx.direct:
-                    weights, arena, X = ctx.weights, saved[0], saved[1]
-                else:
-                    weights, arena, X = saved[:np_], saved[np_], saved[-1]
-                outer._check_input(DY, 'DY')
-                DY = DY.contiguous()
-                bplan, btotal = outer._bwd_plan
-                gplan, gtotal = outer._grad_plan
-                if ctx.pool_set is not None:
-                    DX, barena = ctx.pool_set['DX'], ctx.pool_set['bwd']
-                    garena = ctx.pool_set['grads'] if not outer.__dict__.get('_grad_arenas') else \
-                        outer._next_grad_arena(gtotal, DY.device)
-                else:
-                    DX = torch.empty_like(DY)
-                    barena = torch.empty(max(btotal, 1), dtype=torch.uint8, device=DY.device)
-                    garena = outer._next_grad_arena(gtotal, DY.device)
-                tab = outer._pooled_ptrs if ctx.pool_set is not None else \
-                    (lambda which, plan, a, over: outer._plan_ptrs(plan, a, over))
-                outer._backward_ptrs(DY, tab('grads', gplan, garena, {}), tab('bwd', bplan, barena, {}), weights,
-                                     tab('fwd', outer._fwd_plan[0], arena, ctx.masks), X, DX)
-                g16 = garena[:max(gtotal, 2)].view(outer.torch_dtype)
-                outer._grad_bucket = g16
-                grads = tuple(torch.as_strided(g16, shape, strides, off) for shape, strides, off in outer._grad_views)
-                if outer.enable_debug:
-                    torch.cuda.synchronize()
-                    bwd = outer.views('backward', barena)
-                    for name in outer._bwd_names:
-                        outer.debug[name] = _to_numpy(bwd[name])
-                    for name, g in zip(outer._param_names, grads):
-                        outer.debug['D' + name] = _to_numpy(g)
-                if ctx.direct:
-                    for prm, g in zip(outer.params, grads):
-                        if prm.requires_grad:
-                            prm.grad = g
-                    return DX, None, None
-                return (DX, None, *grads)
-
-        self.encoder_func = EncoderFunction
 
     # ------------------------------------------------------------------ parameters
     def reset_parameters(self):
@@ -330,7 +323,7 @@ class Encoder(torch.nn.Module):
                 _lib.load(self._lib_key).sb_encoder_destroy(self._handle)
             except Exception:  # interpreter shutdown
                 pass
-            self._handle = None
+            self.__dict__['_handle'] = None
 
     def __del__(self):
         self._destroy()
@@ -375,10 +368,8 @@ class Encoder(torch.nn.Module):
             arr = cache[key] = self._plan_ptrs(plan, arena, overrides)
         return arr
 
-    def _graphs_now(self, h, on):
-        """Graph replay pays when the buffers of a pass repeat (raw passes into caller-held arenas); the autograd
-        path allocates fresh arenas per step, where capturing would only cost host time."""
-        on = bool(on and self.__dict__.get('_graphs', True))
+    def _graphs_now(self, h):
+        on = self.__dict__.get('_graphs', True)
         if self.__dict__.get('_graphs_state') != on:
             self._check(_lib.load(self._lib_key).sb_encoder_set_graphs(h, int(on)))
             self._graphs_state = on
@@ -386,7 +377,7 @@ class Encoder(torch.nn.Module):
     def _forward_ptrs(self, X, weights, fwd_ptrs, Y):
         lib = _lib.load(self._lib_key)
         h = self._native(X.device)
-        self._graphs_now(h, _AUTOGRAD_GRAPHS or bool(self.__dict__.get('_pool_n')))
+        self._graphs_now(h)
         mode = _lib.SB_MASK_PHILOX if self.mask_mode == 'philox' else _lib.SB_MASK_EXPLICIT
         stream = ctypes.c_void_p(torch.cuda.current_stream(X.device).cuda_stream)
         self._check(lib.sb_encoder_forward(h, stream, ctypes.c_void_p(X.data_ptr()), self._ptrs(weights), fwd_ptrs,
@@ -396,7 +387,7 @@ class Encoder(torch.nn.Module):
     def _backward_ptrs(self, DY, grad_ptrs, bwd_ptrs, weights, fwd_ptrs, X, DX):
         lib = _lib.load(self._lib_key)
         h = self._native(DY.device)
-        self._graphs_now(h, _AUTOGRAD_GRAPHS or bool(self.__dict__.get('_pool_n')))
+        self._graphs_now(h)
         stream = ctypes.c_void_p(torch.cuda.current_stream(DY.device).cuda_stream)
         self._check(lib.sb_encoder_backward(h, stream, ctypes.c_void_p(DY.data_ptr()), grad_ptrs, bwd_ptrs,
                                            self._ptrs(weights), fwd_ptrs, ctypes.c_void_p(X.data_ptr()),
@@ -426,7 +417,7 @@ class Encoder(torch.nn.Module):
         self._check_raw(X.device, X=X, Y=Y, weights=list(weights), fwd={n: fwd[n] for n in self._fwd_names})
         lib = _lib.load(self._lib_key)
         h = self._native(X.device)
-        self._graphs_now(h, True)
+        self._graphs_now(h)
         mode = _lib.SB_MASK_PHILOX if self.mask_mode == 'philox' else _lib.SB_MASK_EXPLICIT
         stream = ctypes.c_void_p(torch.cuda.current_stream(X.device).cuda_stream)
         wl = list(weights)
@@ -447,7 +438,7 @@ class Encoder(torch.nn.Module):
                         fwd={n: fwd[n] for n in self._fwd_names})
         lib = _lib.load(self._lib_key)
         h = self._native(DY.device)
-        self._graphs_now(h, True)
+        self._graphs_now(h)
         stream = ctypes.c_void_p(torch.cuda.current_stream(DY.device).cuda_stream)
         wl = list(weights)
         self._check(lib.sb_encoder_backward(
@@ -504,9 +495,8 @@ class Encoder(torch.nn.Module):
     def set_buffer_pool(self, n, direct_grads=True):
         """``n`` > 0: the autograd path stops allocating per pass and takes the forward arena, the output, the backward
         arena, the input gradient and the gradient bucket from ``n`` sets of buffers the module owns, used in turn
-        (allocated on first use).  The pointers of a pass then repeat every ``n`` steps, so passes are replayed as
-        CUDA graphs with one launch each instead of some thirty, which is what an input pipeline that feeds the
-        module from a few rotating device buffers wants.  The price: a tensor returned by ``forward`` (or a
+        (allocated on first use): what an input pipeline that feeds the module from a few rotating device buffers
+        wants.  The price: a tensor returned by ``forward`` (or a
         gradient produced by ``backward``) is overwritten ``n`` steps later; copy what must live longer.
         ``direct_grads``: backward sets every parameter's ``.grad`` itself (a view into the pooled bucket, replacing
         what was there) instead of handing sixteen gradients to autograd, which takes a third off the host's time per
@@ -566,7 +556,7 @@ class Encoder(torch.nn.Module):
         return self.__dict__.get('_grad_bucket')
 
     def set_graphs(self, enabled):
-        """Replay passes whose buffers repeat as CUDA graphs (default) or launch every kernel each time."""
+        """Run passes as CUDA graphs with rewritten parameters (default) or launch every kernel each time."""
         self._graphs = bool(enabled)
         self._graphs_state = None
 
@@ -592,5 +582,5 @@ class Encoder(torch.nn.Module):
             anchor = self.__dict__.get('_anchor')
             if anchor is None or anchor.device != X.device:
                 anchor = self._anchor = torch.zeros(1, device=X.device, requires_grad=True)
-            return self.encoder_func.apply(X, anchor, tuple(p.detach() for p in self.params))
-        return self.encoder_func.apply(X, None, *self.params)
+            return _EncoderFunction.apply(self, X, anchor, tuple(p.detach() for p in self.params))
+        return _EncoderFunction.apply(self, X, None, *self.params)
