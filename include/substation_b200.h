@@ -356,6 +356,22 @@ int sb_encoder_forward(sb_encoder* enc, void* stream, const void* x, const void*
 int sb_encoder_backward(sb_encoder* enc, void* stream, const void* dy, void* const* dparams,
                         void* const* bwd, const void* const* params, void* const* fwd,
                         const void* x, void* dx);
+/* The same passes for callers that look at none of the intermediates: attention keeps a log-sum-exp per row and a mask
+ * bit per score in `scratch` instead of the score tensors, and computes the scores again in the backward pass.  BETA,
+ * ALPHA, ATTN_DROP, DATTN_DROP, DBETA and (philox) ATTN_DROP_MASK are neither read nor written, their table entries only
+ * have to be non-null.  sb_encoder_private_bytes gives the two scratch sizes for a mask mode; both are 0 when these
+ * passes do not apply: fusion off, dead stores on, head size other than 64, or layouts the kernels do not read (the
+ * passes themselves then return SB_ERR_UNSUPPORTED for the last two).  A backward pass takes the scratch of its forward
+ * pass, which must have run with keep != 0, and that pass's mask mode; scratch is 16-byte aligned.  Intermediates are kept in
+ * orders of the library's choosing (same sizes); x, y, dy, dx, parameters, their gradients and explicit masks keep the
+ * configured ones. */
+int sb_encoder_private_bytes(sb_encoder* enc, int mask_mode, size_t* forward, size_t* backward);
+int sb_encoder_forward_private(sb_encoder* enc, void* stream, const void* x, const void* const* params,
+                               void* const* fwd, void* y, void* scratch, int keep, int mask_mode, uint64_t seed,
+                               uint64_t offset);
+int sb_encoder_backward_private(sb_encoder* enc, void* stream, const void* dy, void* const* dparams,
+                                void* const* bwd, const void* const* params, void* const* fwd, const void* x, void* dx,
+                                const void* fwd_scratch, void* scratch, int mask_mode);
 /* Per-operator device time of the most recent forward+backward, measured with
  * CUDA events when timing was switched on; writes up to max (name, ms) pairs
  * and returns the count.  While timing is on every operator is also an NVTX range

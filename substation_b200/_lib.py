@@ -97,6 +97,12 @@ SIGNATURES = {
                                    ctypes.c_uint64, ctypes.c_uint64]),
     'sb_encoder_backward': (c_int, [c_void_p, c_void_p, c_void_p, _PP, _PP, _PP, _PP, c_void_p,
                                     c_void_p]),
+    'sb_encoder_private_bytes': (c_int, [c_void_p, c_int, ctypes.POINTER(ctypes.c_size_t),
+                                         ctypes.POINTER(ctypes.c_size_t)]),
+    'sb_encoder_forward_private': (c_int, [c_void_p, c_void_p, c_void_p, _PP, _PP, c_void_p, c_void_p, c_int, c_int,
+                                           ctypes.c_uint64, ctypes.c_uint64]),
+    'sb_encoder_backward_private': (c_int, [c_void_p, c_void_p, c_void_p, _PP, _PP, _PP, _PP, c_void_p, c_void_p,
+                                            c_void_p, c_void_p, c_int]),
     'sb_encoder_set_timing': (c_int, [c_void_p, c_int]),
     'sb_encoder_get_timing': (c_int, [c_void_p, c_int, ctypes.POINTER(c_char_p),
                                       ctypes.POINTER(c_float)]),

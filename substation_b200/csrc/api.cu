@@ -705,7 +705,7 @@ struct sb_encoder {
     long long passes = 0, captures = 0, replays = 0;
     void drop() { slot[0].drop(); slot[1].drop(); }
   };
-  GraphCache graph_fwd, graph_bwd;
+  GraphCache graph_fwd, graph_bwd, graph_fwd_private, graph_bwd_private;
   bool rewriting = false;       // a pass is running that only rewrites a graph's kernel parameters
   cudaStream_t capture_stream = nullptr;
   cudaEvent_t ffn_grads_event = nullptr;   // recorded in backward once the feed-forward gradients are final
@@ -978,6 +978,8 @@ extern "C" int sb_encoder_destroy(sb_encoder* e) {
   if (e->workspace) cudaFree(e->workspace);
   e->graph_fwd.drop();
   e->graph_bwd.drop();
+  e->graph_fwd_private.drop();
+  e->graph_bwd_private.drop();
   if (e->capture_stream) cudaStreamDestroy(e->capture_stream);
   delete e;
   return SB_OK;
@@ -1012,15 +1014,21 @@ extern "C" int sb_encoder_set_graphs(sb_encoder* e, int enabled) {
 extern "C" int sb_encoder_set_ffn_grads_event(sb_encoder* e, void* event) {
   if (!e) return fail(SB_ERR_ARG, "null handle");
   // graphs captured so far record the previous event (or none)
-  if (e->ffn_grads_event != (cudaEvent_t)event) e->graph_bwd.drop();
+  if (e->ffn_grads_event != (cudaEvent_t)event) {
+    e->graph_bwd.drop();
+    e->graph_bwd_private.drop();
+  }
   e->ffn_grads_event = (cudaEvent_t)event;
   return SB_OK;
 }
 
 extern "C" int sb_encoder_graph_stats(sb_encoder* e, long long* captures, long long* replays) {
   if (!e || !captures || !replays) return fail(SB_ERR_ARG, "sb_encoder_graph_stats: null argument");
-  *captures = e->graph_fwd.captures + e->graph_bwd.captures;
-  *replays = e->graph_fwd.replays + e->graph_bwd.replays;
+  *captures = *replays = 0;
+  for (const auto* c : {&e->graph_fwd, &e->graph_bwd, &e->graph_fwd_private, &e->graph_bwd_private}) {
+    *captures += c->captures;
+    *replays += c->replays;
+  }
   return SB_OK;
 }
 
@@ -1067,6 +1075,14 @@ int gather(sb_encoder* e, const void* x, const void* const* params, void* const*
   return SB_OK;
 }
 
+// projection in logical order [P,H,B,J] as the attention launchers take it
+View4 proj_view(const sb_tensor& t) {
+  View4 v;
+  v.p = nullptr; v.vec = 0;
+  v.sH = t.stride[0]; v.sB = t.stride[1]; v.sJ = t.stride[2]; v.sK = t.stride[3];
+  return v;
+}
+
 sb_dropout drop(float p, int mode, uint64_t seed, uint64_t offset) {
   sb_dropout d;
   d.p = p; d.mode = mode; d.seed = seed; d.offset = offset;
@@ -1075,8 +1091,13 @@ sb_dropout drop(float p, int mode, uint64_t seed, uint64_t offset) {
 
 }  // namespace
 
+// `priv`: nobody looks at the intermediates of this pass; attention keeps its own state in priv->scratch.
+struct PrivateForward { void* scratch; bool keep; };
+struct PrivateBackward { const void* fwd_scratch; void* scratch; };
+
 static int forward_pass(sb_encoder* e, void* stream, const void* x, const void* const* params,
-                        void* const* fwd, void* y, int mask_mode, uint64_t seed, uint64_t offset) {
+                        void* const* fwd, void* y, int mask_mode, uint64_t seed, uint64_t offset,
+                        const PrivateForward* priv) {
   if (!e || !y) return fail(SB_ERR_ARG, "sb_encoder_forward: null argument");
   if (mask_mode != SB_MASK_EXPLICIT && mask_mode != SB_MASK_PHILOX)
     return fail(SB_ERR_ARG, "sb_encoder_forward: unknown mask mode");
@@ -1118,8 +1139,17 @@ static int forward_pass(sb_encoder* e, void* stream, const void* x, const void* 
       SB_TRY(sb_attention_input_biases(stream, &in, &bias, &out));
     }
   }
+  if (priv) {
+    e->mark(s, "attention");
+    sb_dropout d = drop(e->p_softmax, mask_mode, seed, offset + 0);
+    Rng rng;
+    SB_TRY(to_rng(&d, &rng));
+    SB_TRY(launch_flash_fwd(s, e->H, e->B, e->S, T[TID("KKQQVV")], slice, proj_view(e->proj), T[TID("GAMMA")],
+                            proj_view(e->logical[TID("GAMMA")]), T[TID("ATTN_DROP_MASK")], 1.f / std::sqrt((float)e->P), rng,
+                            priv->scratch, priv->keep));
+  }
   // F2 + softmax.  K and V views are the J-indexed projections relabelled with K.
-  {
+  if (!priv) {
     sb_tensor beta = v(TID("BETA")), alpha = v(TID("ALPHA"));
     sb_tensor mask = v(TID("ATTN_DROP_MASK")), dr = v(TID("ATTN_DROP"));
     sb_dropout d = drop(e->p_softmax, mask_mode, seed, offset + 0);
@@ -1140,7 +1170,7 @@ static int forward_pass(sb_encoder* e, void* stream, const void* x, const void* 
       SB_TRY(sb_softmax_dropout(stream, &beta, &alpha, &mask, &dr, 1.f, &d));
     }
   }
-  {
+  if (!priv) {
     // one CTA per (head, sample) streams ATTN_DROP once
     int st = SB_ERR_UNSUPPORTED;
     if (e->fuse) {
@@ -1222,7 +1252,7 @@ static int forward_pass(sb_encoder* e, void* stream, const void* x, const void* 
 
 static int backward_pass(sb_encoder* e, void* stream, const void* dy, void* const* dparams,
                          void* const* bwd, const void* const* params, void* const* fwd,
-                         const void* x, void* dx) {
+                         const void* x, void* dx, const PrivateBackward* priv) {
   if (!e || !dy || !dparams || !bwd || !dx) return fail(SB_ERR_ARG, "sb_encoder_backward: null argument");
   cudaStream_t s = (cudaStream_t)stream;
   Ptrs T;
@@ -1316,7 +1346,13 @@ static int backward_pass(sb_encoder* e, void* stream, const void* dy, void* cons
   const float scale = 1.f / std::sqrt((float)e->P);
   void *KK = q_slice(T[TID("KKQQVV")], 0), *QQ = q_slice(T[TID("KKQQVV")], 1), *VV = q_slice(T[TID("KKQQVV")], 2);
   void *DKK = q_slice(T[TID("DKKQQVV")], 0), *DQQ = q_slice(T[TID("DKKQQVV")], 1), *DVV = q_slice(T[TID("DKKQQVV")], 2);
-  {
+  if (priv) {
+    e->mark(s, "attention-backward");
+    SB_TRY(launch_flash_bwd(s, e->H, e->B, e->S, T[TID("KKQQVV")], slice, proj_view(e->proj), T[TID("GAMMA")],
+                            proj_view(e->logical[TID("GAMMA")]), T[TID("DGAMMA")], proj_view(e->logical[TID("DGAMMA")]),
+                            T[TID("DKKQQVV")], slice, proj_view(e->dproj), scale, priv->fwd_scratch, priv->scratch));
+  }
+  if (!priv) {
     sb_tensor alpha = v(TID("ALPHA")), mask = v(TID("ATTN_DROP_MASK")), g = v(TID("DATTN_DROP")), o = v(TID("DBETA"));
     int st = SB_ERR_UNSUPPORTED;
     if (e->fuse) {
@@ -1348,7 +1384,7 @@ static int backward_pass(sb_encoder* e, void* stream, const void* dy, void* cons
       SB_TRY(sb_backward_softmax(stream, &alpha, &mask, &g, &o));
     }
   }
-  {
+  if (!priv) {
     // both projection gradients from one pass over DBETA
     int st = SB_ERR_UNSUPPORTED;
     if (e->fuse) {
@@ -1528,7 +1564,7 @@ int run_pass(sb_encoder* e, sb_encoder::GraphCache& cache, cudaStream_t s, Pass&
 extern "C" int sb_encoder_forward(sb_encoder* e, void* stream, const void* x, const void* const* params,
                                   void* const* fwd, void* y, int mask_mode, uint64_t seed, uint64_t offset) {
   if (!e || !y || !params || !fwd) return fail(SB_ERR_ARG, "sb_encoder_forward: null argument");
-  auto pass = [&](cudaStream_t s) { return forward_pass(e, (void*)s, x, params, fwd, y, mask_mode, seed, offset); };
+  auto pass = [&](cudaStream_t s) { return forward_pass(e, (void*)s, x, params, fwd, y, mask_mode, seed, offset, nullptr); };
   return run_pass(e, e->graph_fwd, (cudaStream_t)stream, pass);
 }
 
@@ -1537,6 +1573,56 @@ extern "C" int sb_encoder_backward(sb_encoder* e, void* stream, const void* dy, 
                                    const void* x, void* dx) {
   if (!e || !dy || !dparams || !bwd || !dx || !params || !fwd)
     return fail(SB_ERR_ARG, "sb_encoder_backward: null argument");
-  auto pass = [&](cudaStream_t s) { return backward_pass(e, (void*)s, dy, dparams, bwd, params, fwd, x, dx); };
+  auto pass = [&](cudaStream_t s) { return backward_pass(e, (void*)s, dy, dparams, bwd, params, fwd, x, dx, nullptr); };
   return run_pass(e, e->graph_bwd, (cudaStream_t)stream, pass);
+}
+
+namespace {
+
+int private_supported(const sb_encoder* e) {
+  if (e->dims[TID("ATTN_DROP_MASK")] != "HBJK" ||
+      flash_supported(e->H, e->B, e->S, e->P, proj_view(e->proj), proj_view(e->dproj), proj_view(e->logical[TID("GAMMA")]),
+                      proj_view(e->logical[TID("DGAMMA")])) != SB_OK)
+    return fail(SB_ERR_UNSUPPORTED, "private passes need head size 64, score masks stored as HBJK and projections with unit "
+                                    "stride along the head or the sequence dim");
+  return SB_OK;
+}
+
+}  // namespace
+
+extern "C" int sb_encoder_private_bytes(sb_encoder* e, int mask_mode, size_t* forward, size_t* backward) {
+  if (!e || !forward || !backward) return fail(SB_ERR_ARG, "sb_encoder_private_bytes: null argument");
+  (void)mask_mode;
+  *forward = *backward = 0;
+  if (!e->fuse || e->dead_stores || private_supported(e) != SB_OK) return SB_OK;
+  FlashScratch f;
+  flash_scratch(e->H, e->B, e->S, flash_padded(proj_view(e->proj), e->S), flash_padded(proj_view(e->logical[TID("DGAMMA")]), e->S), &f);
+  *forward = f.fwd_bytes;
+  *backward = f.bwd_bytes;
+  return SB_OK;
+}
+
+extern "C" int sb_encoder_forward_private(sb_encoder* e, void* stream, const void* x, const void* const* params,
+                                          void* const* fwd, void* y, void* scratch, int keep, int mask_mode,
+                                          uint64_t seed, uint64_t offset) {
+  if (!e || !x || !y || !params || !fwd || !scratch) return fail(SB_ERR_ARG, "sb_encoder_forward_private: null argument");
+  if (!aligned(scratch, 16)) return fail(SB_ERR_ALIGNMENT, "sb_encoder_forward_private: scratch is not 16-byte aligned");
+  SB_TRY(private_supported(e));
+  const PrivateForward priv{scratch, keep != 0};
+  auto pass = [&](cudaStream_t s) { return forward_pass(e, (void*)s, x, params, fwd, y, mask_mode, seed, offset, &priv); };
+  return run_pass(e, e->graph_fwd_private, (cudaStream_t)stream, pass);
+}
+
+extern "C" int sb_encoder_backward_private(sb_encoder* e, void* stream, const void* dy, void* const* dparams,
+                                           void* const* bwd, const void* const* params, void* const* fwd,
+                                           const void* x, void* dx, const void* fwd_scratch, void* scratch, int mask_mode) {
+  if (!e || !dy || !dparams || !bwd || !x || !dx || !params || !fwd || !fwd_scratch || !scratch)
+    return fail(SB_ERR_ARG, "sb_encoder_backward_private: null argument");
+  if (!aligned(fwd_scratch, 16) || !aligned(scratch, 16))
+    return fail(SB_ERR_ALIGNMENT, "sb_encoder_backward_private: scratch is not 16-byte aligned");
+  (void)mask_mode;
+  SB_TRY(private_supported(e));
+  const PrivateBackward priv{fwd_scratch, scratch};
+  auto pass = [&](cudaStream_t s) { return backward_pass(e, (void*)s, dy, dparams, bwd, params, fwd, x, dx, &priv); };
+  return run_pass(e, e->graph_bwd_private, (cudaStream_t)stream, pass);
 }

@@ -683,6 +683,7 @@ splitk_reduce_kernel(const float* __restrict__ ws, int splits, long long batch, 
 #include "gemm_pair_splitk.cuh"
 #include "attn_fused.cuh"
 #include "score_contract.cuh"
+#include "flash_attn.cuh"
 #include "peak_probe.cuh"
 
 // ---- host side ------------------------------------------------------------
@@ -1307,6 +1308,153 @@ int launch_score_contract(cudaStream_t s, Dims4 d, int P, View4 scores, const Vi
   SB_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(scon::score_contract_kernel), 232448));
   const unsigned grid = (unsigned)std::min<long long>(batch, sm_count());
   SB_LAUNCH_OK(launch_k(scon::score_contract_kernel, grid, kTcThreads, smem, s, ms, mx, my, p));
+  return SB_OK;
+}
+
+namespace {
+
+// [P,H,B,rows] projection (View4 fields hold the P,H,B,row strides) as rows of units h * B + b.
+struct UnitView { long long sP, sU, sRow; };
+bool unit_view(const View4& v, int H, int B, UnitView* o) {
+  if (H > 1 && B > 1 && v.sB != v.sJ * B) return false;
+  o->sP = v.sH; o->sU = B > 1 ? v.sJ : v.sB; o->sRow = v.sK;
+  return true;
+}
+// Tensor map of a projection the flash kernels read in 64 x 64 boxes: `jc` when the rows are the unit-stride index.
+bool flash_map(const void* ptr, const UnitView& v, int units, int L, CUtensorMap* map, int* jc, int* swap, std::string* why) {
+  OperandMap m;
+  if (!make_operand_map(ptr, L, 64, units, v.sRow, v.sP, v.sU, 64, &m, why)) return false;
+  *map = m.map; *jc = m.mn; *swap = m.swap;
+  return true;
+}
+long long pad8(long long n) { return (n + 7) / 8 * 8; }
+size_t align256(size_t n) { return (n + 255) / 256 * 256; }
+
+}  // namespace
+
+// Rows of the projections are the unit-stride index and not 16 bytes apart: the kernels read a padded copy.
+bool flash_padded(const View4& v, int L) { return v.sK == 1 && v.sH != 1 && L % 8 != 0; }
+
+int flash_supported(int H, int B, int L, int P, View4 proj, View4 dproj, View4 gamma, View4 dgamma) {
+  UnitView u;
+  for (const View4* v : {&proj, &dproj, &gamma, &dgamma})
+    if (!unit_view(*v, H, B, &u)) return SB_ERR_UNSUPPORTED;
+  for (const View4* v : {&proj, &dgamma}) {
+    if (v->sH != 1 && v->sK != 1) return SB_ERR_UNSUPPORTED;
+    if (v->sH == 1 && ((v->sK | v->sJ | v->sB) & 7)) return SB_ERR_UNSUPPORTED;
+  }
+  if (P != 64 || L < 1 || (long long)H * B * ((L + 31) / 32) > 0x3fffffffLL) return SB_ERR_UNSUPPORTED;
+  return SB_OK;
+}
+
+void flash_scratch(int H, int B, int L, bool pad_proj, bool pad_dgamma, FlashScratch* f) {
+  const size_t units = (size_t)H * B, nb = (L + 127) / 128;
+  f->bits = align256(units * L * sizeof(float));
+  f->pad = f->bits + align256(units * nb * L * 16);
+  f->fwd_bytes = f->pad + (pad_proj ? align256(192 * units * pad8(L) * 2) : 0);
+  f->dpad = align256(units * L * sizeof(float));
+  f->bwd_bytes = f->dpad + (pad_dgamma ? align256(64 * units * pad8(L) * 2) : 0);
+}
+
+int launch_flash_fwd(cudaStream_t s, int H, int B, int L, const void* kqv, long long slice, View4 proj, void* gamma, View4 gv,
+                     const void* mask, float scale, Rng rng, void* scratch, bool keep) {
+  std::call_once(g_encode_once, load_encode);
+  if (!g_encode) return fail(SB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+  const int units = H * B;
+  FlashScratch f;
+  const bool pad = flash_padded(proj, L);
+  flash_scratch(H, B, L, pad, false, &f);
+  char* sc = reinterpret_cast<char*>(scratch);
+  UnitView v, o;
+  if (!unit_view(proj, H, B, &v) || !unit_view(gv, H, B, &o)) return fail(SB_ERR_UNSUPPORTED, "attention: head and sample dims do not collapse");
+  const sb_half* base = reinterpret_cast<const sb_half*>(kqv);
+  if (pad) {
+    sb_half* dst = reinterpret_cast<sb_half*>(sc + f.pad);
+    const unsigned grid = (unsigned)std::min<long long>((192ll * units + 7) / 8, (long long)sm_count() * 8);
+    SB_LAUNCH_OK(launch_k(flash::pad_projections_kernel, grid, 256, 0, s, base, slice, v.sP, v.sU, dst, units, L, (int)pad8(L)));
+    base = dst;
+    v.sRow = 1; v.sU = pad8(L); v.sP = v.sU * units;
+    slice = 64 * v.sP;
+  }
+  flash::FwdParams p;
+  memset(&p, 0, sizeof(p));
+  std::string why;
+  CUtensorMap mk, mq, mv;
+  if (!flash_map(base, v, units, L, &mk, &p.jc, &p.k_swap, &why) || !flash_map(base + slice, v, units, L, &mq, &p.jc, &p.q_swap, &why) ||
+      !flash_map(base + 2 * slice, v, units, L, &mv, &p.jc, &p.v_swap, &why))
+    return fail(SB_ERR_UNSUPPORTED, "attention, projections: " + why);
+  p.L = L; p.nb = (L + 127) / 128; p.items = units * p.nb;
+  p.c2 = scale * 1.4426950408889634f;
+  p.rng = rng;
+  p.mask = reinterpret_cast<const uint8_t*>(mask);
+  if (keep) { p.lse = reinterpret_cast<float*>(sc); p.bits = reinterpret_cast<uint4*>(sc + f.bits); }
+  p.out = reinterpret_cast<sb_half*>(gamma);
+  p.o_sU = o.sU; p.o_sRow = o.sRow; p.o_sP = o.sP;
+  const bool none = rng.philox && rng.thr == 0;
+  auto kernel = none ? flash::flash_fwd_kernel<flash::kNoDrop>
+                     : rng.philox && L % 8 == 0 ? flash::flash_fwd_kernel<flash::kPhilox> : flash::flash_fwd_kernel<flash::kAnyMask>;
+  SB_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), flash::kFwdSmem));
+  const unsigned grid = (unsigned)std::min<long long>(p.items, 2ll * sm_count());
+  SB_LAUNCH_OK(launch_k(kernel, grid, flash::kFwdThreads, flash::kFwdSmem, s, mq, mk, mv, p));
+  return SB_OK;
+}
+
+int launch_flash_bwd(cudaStream_t s, int H, int B, int L, const void* kqv, long long slice, View4 proj, const void* gamma, View4 gv,
+                     const void* dgamma, View4 dgv, void* dkqv, long long dslice, View4 dproj, float scale, const void* fwd_scratch,
+                     void* bwd_scratch) {
+  std::call_once(g_encode_once, load_encode);
+  if (!g_encode) return fail(SB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+  const int units = H * B;
+  FlashScratch f;
+  const bool pad = flash_padded(proj, L), dpad = flash_padded(dgv, L);
+  flash_scratch(H, B, L, pad, dpad, &f);
+  const char* fs = reinterpret_cast<const char*>(fwd_scratch);
+  char* bs = reinterpret_cast<char*>(bwd_scratch);
+  UnitView v, o, g, d;
+  if (!unit_view(proj, H, B, &v) || !unit_view(gv, H, B, &o) || !unit_view(dgv, H, B, &g) || !unit_view(dproj, H, B, &d))
+    return fail(SB_ERR_UNSUPPORTED, "attention: head and sample dims do not collapse");
+  const sb_half* base = reinterpret_cast<const sb_half*>(kqv);
+  if (pad) {
+    base = reinterpret_cast<const sb_half*>(fs + f.pad);
+    v.sRow = 1; v.sU = pad8(L); v.sP = v.sU * units;
+    slice = 64 * v.sP;
+  }
+  flash::DsumParams q;
+  memset(&q, 0, sizeof(q));
+  q.g = reinterpret_cast<const sb_half*>(dgamma); q.g_sP = g.sP; q.g_sU = g.sU; q.g_sRow = g.sRow;
+  q.o = reinterpret_cast<const sb_half*>(gamma); q.o_sP = o.sP; q.o_sU = o.sU; q.o_sRow = o.sRow;
+  q.dsum = reinterpret_cast<float*>(bs);
+  q.pad = dpad ? reinterpret_cast<sb_half*>(bs + f.dpad) : nullptr;
+  q.units = units; q.L = L; q.Lp = (int)pad8(L); q.blocks_j = (L + 31) / 32;
+  SB_LAUNCH_OK(launch_k(flash::dsum_kernel, (unsigned)((long long)units * q.blocks_j), 256, 0, s, q));
+  const void* gptr = dgamma;
+  if (dpad) {
+    gptr = q.pad;
+    g.sRow = 1; g.sU = q.Lp; g.sP = g.sU * units;
+  }
+  flash::BwdParams p;
+  memset(&p, 0, sizeof(p));
+  std::string why;
+  CUtensorMap mk, mq, mv, mg;
+  if (!flash_map(base, v, units, L, &mk, &p.jc, &p.k_swap, &why) || !flash_map(base + slice, v, units, L, &mq, &p.jc, &p.q_swap, &why) ||
+      !flash_map(base + 2 * slice, v, units, L, &mv, &p.jc, &p.v_swap, &why) || !flash_map(gptr, g, units, L, &mg, &p.g_jc, &p.g_swap, &why))
+    return fail(SB_ERR_UNSUPPORTED, "attention backward, operands: " + why);
+  p.L = L; p.nb = (L + 127) / 128; p.units = units;
+  p.both = p.nb == 1 ? 1 : 0;
+  p.first_q = units * p.nb;
+  p.items = p.both ? p.first_q : 2 * p.first_q;
+  p.scale = scale;
+  p.c2 = scale * 1.4426950408889634f;
+  p.lse = reinterpret_cast<const float*>(fs);
+  p.bits = reinterpret_cast<const uint4*>(fs + f.bits);
+  p.dsum = q.dsum;
+  sb_half* dk = reinterpret_cast<sb_half*>(dkqv);
+  p.dk = dk; p.dq = dk + dslice; p.dv = dk + 2 * dslice;
+  p.d_sU = d.sU; p.d_sRow = d.sRow; p.d_sP = d.sP;
+  static_assert(flash::kBwdSmem <= 232448, "shared memory of the attention backward kernel");
+  SB_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(flash::flash_bwd_kernel), flash::kBwdSmem));
+  const unsigned grid = (unsigned)std::min<long long>(p.items, sm_count());
+  SB_LAUNCH_OK(launch_k(flash::flash_bwd_kernel, grid, flash::kBwdThreads, flash::kBwdSmem, s, mq, mk, mv, mg, p));
   return SB_OK;
 }
 

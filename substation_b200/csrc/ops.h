@@ -70,6 +70,22 @@ int launch_attn_scores_bwd(cudaStream_t s, Dims4 d, int P, View4 dgamma, View4 v
 int launch_score_contract(cudaStream_t s, Dims4 d, int P, View4 scores, const View4* x, const View4* out_r, const View4* y,
                           const View4* out_c, float alpha);
 
+// Attention that keeps a log-sum-exp per row and a mask bit per score instead of the score tensors (flash_attn.cuh).
+// kqv / dkqv: the stacked K, Q, V projections and their gradients, `slice` elements apart; View4 convention as above.
+// SB_ERR_UNSUPPORTED (from flash_supported) when head size or layouts do not qualify.
+struct FlashScratch {
+  size_t bits, pad, fwd_bytes;   // forward: log-sum-exps at 0, then mask bits, then padded projections
+  size_t dpad, bwd_bytes;        // backward: row sums at 0, then padded DGAMMA
+};
+int flash_supported(int H, int B, int L, int P, View4 proj, View4 dproj, View4 gamma, View4 dgamma);
+bool flash_padded(const View4& v, int L);
+void flash_scratch(int H, int B, int L, bool pad_proj, bool pad_dgamma, FlashScratch* f);
+int launch_flash_fwd(cudaStream_t s, int H, int B, int L, const void* kqv, long long slice, View4 proj, void* gamma, View4 gv,
+                     const void* mask, float scale, Rng rng, void* scratch, bool keep);
+int launch_flash_bwd(cudaStream_t s, int H, int B, int L, const void* kqv, long long slice, View4 proj, const void* gamma, View4 gv,
+                     const void* dgamma, View4 dgv, void* dkqv, long long dslice, View4 dproj, float scale, const void* fwd_scratch,
+                     void* bwd_scratch);
+
 // Contractions -----------------------------------------------------------------
 struct GemmProblem {
   long long batch, M, N, K;

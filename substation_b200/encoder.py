@@ -43,10 +43,11 @@ def _to_numpy(t):
 
 class _EncoderFunction(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, outer, X, anchor, *weights):
+    def forward(ctx, outer, X, keep, anchor, *weights):
         ctx.outer = outer
         # Hot path: one arena per pass, pointers computed from the plan's offsets; tensor views
         # over the arena are only built when somebody asks for them (debug, or a caller of views()).
+        # ``keep``: a backward pass may follow.
         # ``anchor`` is None on the ordinary path (``weights`` are the sixteen parameters, and autograd routes
         # their gradients).  With a buffer pool it is a one-element leaf that keeps the node in the graph,
         # ``weights`` is ONE tuple of detached parameters that autograd does not look into, and backward
@@ -57,8 +58,12 @@ class _EncoderFunction(torch.autograd.Function):
         outer._check_input(X, 'X')
         X = X.contiguous()
         weights = tuple(w if w.is_contiguous() else w.contiguous() for w in weights)
-        plan, total = outer._fwd_plan
-        pooled = outer._pool_set(X) if outer.__dict__.get('_pool_n') else None
+        # Nobody sees the intermediates of this pass: attention may keep its own, far smaller, state (enable_debug and
+        # keep_all_intermediates rule it out, as does an operator-by-operator table of times).
+        private = outer._private_plans(X.device)
+        ctx.private = private
+        plan, total = private['fwd'] if private else outer._fwd_plan
+        pooled = outer._pool_set(X, private) if outer.__dict__.get('_pool_n') else None
         if pooled is not None:
             Y, arena = pooled['Y'], pooled['fwd']
             ctx.pool_set = pooled
@@ -67,9 +72,10 @@ class _EncoderFunction(torch.autograd.Function):
             arena = torch.empty(max(total, 1), dtype=torch.uint8, device=X.device)
             ctx.pool_set = None
         over = outer._explicit_masks(X.device) if outer.mask_mode == 'explicit' else {}
-        ptrs = outer._pooled_ptrs('fwd', plan, arena, over) if pooled is not None else \
+        ptrs = outer._pooled_ptrs('private_fwd' if private else 'fwd', plan, arena, over) if pooled is not None else \
             outer._plan_ptrs(plan, arena, over)
-        outer._forward_ptrs(X, weights, ptrs, Y)
+        scratch = arena.data_ptr() + private['fwd_scratch'] if private else None
+        outer._forward_ptrs(X, weights, ptrs, Y, scratch, keep)
         if ctx.direct:
             ctx.weights = weights
             ctx.save_for_backward(arena, X)
@@ -97,7 +103,9 @@ class _EncoderFunction(torch.autograd.Function):
             weights, arena, X = saved[:np_], saved[np_], saved[-1]
         outer._check_input(DY, 'DY')
         DY = DY.contiguous()
-        bplan, btotal = outer._bwd_plan
+        private = ctx.private
+        fplan = private['fwd'][0] if private else outer._fwd_plan[0]
+        bplan, btotal = private['bwd'] if private else outer._bwd_plan
         gplan, gtotal = outer._grad_plan
         if ctx.pool_set is not None:
             DX, barena = ctx.pool_set['DX'], ctx.pool_set['bwd']
@@ -109,8 +117,11 @@ class _EncoderFunction(torch.autograd.Function):
             garena = outer._next_grad_arena(gtotal, DY.device)
         tab = outer._pooled_ptrs if ctx.pool_set is not None else \
             (lambda which, plan, a, over: outer._plan_ptrs(plan, a, over))
-        outer._backward_ptrs(DY, tab('grads', gplan, garena, {}), tab('bwd', bplan, barena, {}), weights,
-                             tab('fwd', outer._fwd_plan[0], arena, ctx.masks), X, DX)
+        outer._backward_ptrs(DY, tab('grads', gplan, garena, {}),
+                             tab('private_bwd' if private else 'bwd', bplan, barena, {}), weights,
+                             tab('private_fwd' if private else 'fwd', fplan, arena, ctx.masks), X, DX,
+                             (arena.data_ptr() + private['fwd_scratch'], barena.data_ptr() + private['bwd_scratch'],
+                              private['mask_mode']) if private else None)
         g16 = garena[:max(gtotal, 2)].view(outer.torch_dtype)
         outer._grad_bucket = g16
         grads = tuple(torch.as_strided(g16, shape, strides, off) for shape, strides, off in outer._grad_views)
@@ -125,8 +136,8 @@ class _EncoderFunction(torch.autograd.Function):
             for prm, g in zip(outer.params, grads):
                 if prm.requires_grad:
                     prm.grad = g
-            return None, DX, None, None
-        return (None, DX, None, *grads)
+            return None, DX, None, None, None
+        return (None, DX, None, None, *grads)
 
 
 class Encoder(torch.nn.Module):
@@ -374,21 +385,59 @@ class Encoder(torch.nn.Module):
             self._check(_lib.load(self._lib_key).sb_encoder_set_graphs(h, int(on)))
             self._graphs_state = on
 
-    def _forward_ptrs(self, X, weights, fwd_ptrs, Y):
+    # attention intermediates a private pass does without
+    _SCORES = frozenset(('BETA', 'ALPHA', 'ATTN_DROP', 'ATTN_DROP_MASK', 'DATTN_DROP', 'DBETA'))
+
+    def _private_plans(self, device):
+        """Arena plans of a pass whose intermediates nobody looks at (score tensors without storage, the library's
+        scratch behind the others), or None where the library has no such pass for this configuration."""
+        if self.enable_debug or self.keep_all_intermediates or self.profiling:
+            return None
+        h = self._native(device)
+        mode = _lib.SB_MASK_PHILOX if self.mask_mode == 'philox' else _lib.SB_MASK_EXPLICIT
+        nf, nb = ctypes.c_size_t(0), ctypes.c_size_t(0)
+        self._check(_lib.load(self._lib_key).sb_encoder_private_bytes(h, mode, ctypes.byref(nf), ctypes.byref(nb)))
+        if nf.value == 0:
+            return None
+        key = (nf.value, nb.value, mode)
+        cached = self.__dict__.get('_private')
+        if cached is None or cached['key'] != key:
+            cached = {'key': key, 'mask_mode': mode}
+            for which, entries, extra in (('fwd', self.layouts['forward_interm'], nf.value),
+                                          ('bwd', self.layouts['backward_interm'], nb.value)):
+                plan, off = [], 0
+                for name, shape, dtype, _, nbytes in self._plan(entries)[0]:
+                    n = 0 if name in self._SCORES else nbytes
+                    plan.append((name, shape, dtype, off if n else 0, n))
+                    off += _round_up(n)
+                cached[which], cached[which + '_scratch'] = (plan, off + extra), off
+            self._private = cached
+        return cached
+
+    def _forward_ptrs(self, X, weights, fwd_ptrs, Y, scratch=None, keep=True):
         lib = _lib.load(self._lib_key)
         h = self._native(X.device)
         self._graphs_now(h)
         mode = _lib.SB_MASK_PHILOX if self.mask_mode == 'philox' else _lib.SB_MASK_EXPLICIT
         stream = ctypes.c_void_p(torch.cuda.current_stream(X.device).cuda_stream)
+        if scratch is not None:
+            self._check(lib.sb_encoder_forward_private(h, stream, X.data_ptr(), self._ptrs(weights), fwd_ptrs, Y.data_ptr(),
+                                                       scratch, int(keep), mode, self.seed, self.philox_offset))
+            self.philox_offset += 4
+            return
         self._check(lib.sb_encoder_forward(h, stream, ctypes.c_void_p(X.data_ptr()), self._ptrs(weights), fwd_ptrs,
                                           ctypes.c_void_p(Y.data_ptr()), mode, self.seed, self.philox_offset))
         self.philox_offset += 4
 
-    def _backward_ptrs(self, DY, grad_ptrs, bwd_ptrs, weights, fwd_ptrs, X, DX):
+    def _backward_ptrs(self, DY, grad_ptrs, bwd_ptrs, weights, fwd_ptrs, X, DX, scratch=None):
         lib = _lib.load(self._lib_key)
         h = self._native(DY.device)
         self._graphs_now(h)
         stream = ctypes.c_void_p(torch.cuda.current_stream(DY.device).cuda_stream)
+        if scratch is not None:
+            self._check(lib.sb_encoder_backward_private(h, stream, DY.data_ptr(), grad_ptrs, bwd_ptrs, self._ptrs(weights),
+                                                        fwd_ptrs, X.data_ptr(), DX.data_ptr(), *scratch))
+            return
         self._check(lib.sb_encoder_backward(h, stream, ctypes.c_void_p(DY.data_ptr()), grad_ptrs, bwd_ptrs,
                                            self._ptrs(weights), fwd_ptrs, ctypes.c_void_p(X.data_ptr()),
                                            ctypes.c_void_p(DX.data_ptr())))
@@ -447,6 +496,50 @@ class Encoder(torch.nn.Module):
             self._ptrs([bwd[n] for n in self._bwd_names]),
             self._ptrs(wl), self._ptrs([fwd[n] for n in self._fwd_names]),
             ctypes.c_void_p(X.data_ptr()), ctypes.c_void_p(DX.data_ptr())))
+        return DX
+
+    def private_arena_bytes(self, device):
+        """(forward, backward) arena bytes of passes whose intermediates nobody looks at (``forward_private``), or None
+        where such passes do not apply: ``enable_debug``, ``keep_all_intermediates``, ``profiling``, ``fuse=False``,
+        a head size other than 64."""
+        with torch.cuda.device(device):
+            plans = self._private_plans(torch.device('cuda', torch.cuda.current_device()))
+        return None if plans is None else (plans['fwd'][1], plans['bwd'][1])
+
+    def _private_arena(self, plans, which, arena):
+        if arena.dtype != torch.uint8 or not arena.is_contiguous() or arena.numel() < plans[which][1] or arena.data_ptr() % 16:
+            raise ValueError(f'arena must be a contiguous, 16-byte aligned uint8 tensor of at least {plans[which][1]} bytes')
+        return self._plan_ptrs(plans[which][0], arena, self._explicit_masks(arena.device)
+                               if which == 'fwd' and self.mask_mode == 'explicit' else None), \
+            arena.data_ptr() + plans[which + '_scratch']
+
+    def forward_private(self, X, weights, arena, Y):
+        """One forward pass that keeps what its backward pass needs in ``arena`` (one uint8 tensor of
+        ``private_arena_bytes``), in an order of the library's choosing: no score tensors.  Buffers as ``forward_raw``."""
+        self._check_input(X, 'X')
+        self._check_input(Y, 'Y')
+        self._check_raw(X.device, X=X, Y=Y, weights=list(weights), arena=arena)
+        plans = self._private_plans(X.device)
+        if plans is None:
+            raise RuntimeError('private passes do not apply to this configuration (see private_arena_bytes)')
+        ptrs, scratch = self._private_arena(plans, 'fwd', arena)
+        self._forward_ptrs(X, list(weights), ptrs, Y, scratch, True)
+        return Y
+
+    def backward_private(self, DY, grads, barena, weights, arena, X, DX):
+        """The backward pass of ``forward_private``; ``grads``: name -> preallocated tensor."""
+        self._check_input(DY, 'DY')
+        self._check_input(DX, 'DX')
+        self._check_input(X, 'X')
+        self._check_raw(DY.device, DY=DY, DX=DX, X=X, weights=list(weights), arena=arena, barena=barena,
+                        grads={n: grads[n] for n in self._param_names})
+        plans = self._private_plans(DY.device)
+        if plans is None:
+            raise RuntimeError('private passes do not apply to this configuration (see private_arena_bytes)')
+        fptrs, fscratch = self._private_arena(plans, 'fwd', arena)
+        bptrs, bscratch = self._private_arena(plans, 'bwd', barena)
+        self._backward_ptrs(DY, self._ptrs([grads[n] for n in self._param_names]), bptrs, list(weights), fptrs, X, DX,
+                            (fscratch, bscratch, plans['mask_mode']))
         return DX
 
     def op_times(self):
@@ -509,19 +602,23 @@ class Encoder(torch.nn.Module):
         self._pool_turn = 0
         self._ptr_cache = {}
 
-    def _pool_set(self, X):
+    def _pool_set(self, X, private=None):
+        fwd, bwd = (private['fwd'][1], private['bwd'][1]) if private else (self._fwd_plan[1], self._bwd_plan[1])
         if len(self._pool) < self._pool_n:
             dev = X.device
             self._pool.append({
                 'Y': torch.empty_like(X), 'DX': torch.empty_like(X),
-                'fwd': torch.empty(max(self._fwd_plan[1], 1), dtype=torch.uint8, device=dev),
-                'bwd': torch.empty(max(self._bwd_plan[1], 1), dtype=torch.uint8, device=dev),
+                'fwd': torch.empty(max(fwd, 1), dtype=torch.uint8, device=dev),
+                'bwd': torch.empty(max(bwd, 1), dtype=torch.uint8, device=dev),
                 'grads': torch.empty(max(self._grad_plan[1], 2), dtype=torch.uint8, device=dev)})
             return self._pool[-1]
         s = self._pool[self._pool_turn % self._pool_n]
         self._pool_turn += 1
         if s['Y'].device != X.device:
             raise ValueError('the buffer pool lives on another device than the input; call set_buffer_pool again')
+        for which, need in (('fwd', fwd), ('bwd', bwd)):   # a pass of the other kind (fusion was switched) came first
+            if s[which].numel() < need:
+                s[which] = torch.empty(need, dtype=torch.uint8, device=X.device)
         return s
 
     def set_grad_arenas(self, arenas):
@@ -582,5 +679,6 @@ class Encoder(torch.nn.Module):
             anchor = self.__dict__.get('_anchor')
             if anchor is None or anchor.device != X.device:
                 anchor = self._anchor = torch.zeros(1, device=X.device, requires_grad=True)
-            return _EncoderFunction.apply(self, X, anchor, tuple(p.detach() for p in self.params))
-        return _EncoderFunction.apply(self, X, None, *self.params)
+            return _EncoderFunction.apply(self, X, True, anchor, tuple(p.detach() for p in self.params))
+        keep = torch.is_grad_enabled() and (X.requires_grad or any(p.requires_grad for p in self.params))
+        return _EncoderFunction.apply(self, X, keep, None, *self.params)

@@ -2,8 +2,9 @@
 data-parallel gradient reduction overlapped with the rest of backward.
 
 The reference times one layer (pytorch_module/run_encoder.py:345-383); a BERT-large
-encoder is 24 of them with independent weights.  Forward keeps every layer's
-intermediates alive (one arena per layer, allocated once and reused every step);
+encoder is 24 of them with independent weights.  Forward keeps what each layer's
+backward needs alive (one arena per layer, allocated once and reused every step; with
+``keep_all_intermediates`` every named intermediate, as views in ``fwd`` and ``bwd``);
 backward walks the layers in reverse with ONE shared arena for backward
 intermediates, writes layer l's 12 parameter gradients into bucket l and starts
 its sum-allreduce at once, so the reduction of layer l runs beside the backward of
@@ -21,14 +22,14 @@ from .encoder import Encoder
 class EncoderStack:
     def __init__(self, num_layers, batch_size, max_seq_len, num_heads, embedding_size, layouts,
                  dropout_p=0.1, device='cuda', mask_mode='philox', seed=0, activation='relu',
-                 weight_std=0.02, group=None, dtype=torch.float16):
+                 weight_std=0.02, group=None, dtype=torch.float16, keep_all_intermediates=None):
         self.device = torch.device(device)
         self.layers = []
         gen = torch.Generator(device=self.device).manual_seed(seed)
         for l in range(num_layers):
             enc = Encoder('', batch_size, max_seq_len, num_heads, embedding_size, layouts, dtype,
                           dropout_p, dropout_p, dropout_p, dropout_p, mask_mode=mask_mode, seed=seed + l,
-                          activation=activation).to(self.device)
+                          activation=activation, keep_all_intermediates=keep_all_intermediates).to(self.device)
             with torch.no_grad():
                 for (name, _), prm in zip(layouts['params'], enc.params):
                     if name in ('WKQV', 'WO', 'LINW1', 'LINW2'):
@@ -42,9 +43,15 @@ class EncoderStack:
         self.table = L.validate(layouts)
         shape_x = L.shape_of(self.table['X'], e0.sizes)
         self.weights = [[p.detach() for p in enc.params] for enc in self.layers]
-        self.fwd = [enc.views('forward', torch.empty(enc.arena_bytes('forward'), dtype=torch.uint8, device=self.device))
-                    for enc in self.layers]
-        self.bwd = e0.views('backward', torch.empty(e0.arena_bytes('backward'), dtype=torch.uint8, device=self.device))
+        # private passes (no score tensors in memory) unless somebody wants to look at the intermediates
+        sizes = e0.private_arena_bytes(self.device)
+        self.private = sizes is not None
+        nf, nb = sizes or e0.intermediate_bytes()
+        self.arena_bytes = (nf, nb)
+        arenas = [torch.empty(nf, dtype=torch.uint8, device=self.device) for _ in self.layers]
+        barena = torch.empty(nb, dtype=torch.uint8, device=self.device)
+        self.fwd = arenas if self.private else [enc.views('forward', a) for enc, a in zip(self.layers, arenas)]
+        self.bwd = barena if self.private else e0.views('backward', barena)
         # activations between layers: acts[l] is the input of layer l, acts[-1] the output
         self.acts = [torch.empty(shape_x, dtype=dtype, device=self.device) for _ in range(num_layers + 1)]
         self.dacts = [torch.empty(shape_x, dtype=dtype, device=self.device) for _ in range(2)]
@@ -56,12 +63,13 @@ class EncoderStack:
 
     def memory_bytes(self):
         e0 = self.layers[0]
-        return (len(self.layers) * (e0.arena_bytes('forward') + e0.arena_bytes('grads')) + e0.arena_bytes('backward'))
+        return len(self.layers) * (self.arena_bytes[0] + e0.arena_bytes('grads')) + self.arena_bytes[1]
 
     def forward(self, X):
         self.acts[0].copy_(X)
         for l, enc in enumerate(self.layers):
-            enc.forward_raw(self.acts[l], self.weights[l], self.fwd[l], self.acts[l + 1])
+            run = enc.forward_private if self.private else enc.forward_raw
+            run(self.acts[l], self.weights[l], self.fwd[l], self.acts[l + 1])
         return self.acts[-1]
 
     def backward(self, DY, trace=None):
@@ -82,7 +90,8 @@ class EncoderStack:
         for l in range(len(self.layers) - 1, -1, -1):
             self.reducer.wait(l)                         # bucket l free again (previous step's reduction done)
             out = self.dacts[l & 1]
-            self.layers[l].backward_raw(cur, self.grads[l], self.bwd, self.weights[l], self.fwd[l], self.acts[l], out)
+            run = self.layers[l].backward_private if self.private else self.layers[l].backward_raw
+            run(cur, self.grads[l], self.bwd, self.weights[l], self.fwd[l], self.acts[l], out)
             if tracing:
                 done = torch.cuda.Event(enable_timing=True)
                 done.record()

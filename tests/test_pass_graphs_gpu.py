@@ -45,8 +45,8 @@ def test_rewritten_graphs_match_plain_launches(mask_mode, B, S):
         keep.append(got)                                # nothing is freed: no buffer comes back
         assert all(torch.equal(a, b) for a, b in zip(*got)), step
     captures, runs = encs[0].graph_stats()
-    # two graphs per direction, captured again after the switch (forward only where it changes the kernels: at S = 40
-    # none are fused to begin with); of 12 forward and 9 backward passes the first of each is launched plainly
-    assert captures == (8 if S % 64 == 0 else 6) and runs == 12 + 9 - 2 - captures
+    # passes without and with score tensors (before and after the switch) have graphs of their own, two per direction:
+    # forward 8 + 4 passes, backward 6 + 3, the first of each kind launched plainly
+    assert captures == 2 + 2 + 2 + 1 and runs == 12 + 9 - 4 - captures
     assert encs[1].graph_stats() == (0, 0)
     assert ops.device_error() == 0

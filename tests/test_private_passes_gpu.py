@@ -1,0 +1,119 @@
+"""Passes whose intermediates nobody looks at (autograd's default path: attention without score tensors, activations in
+their logical order, act' in a contraction's epilogue) against passes that keep every intermediate, same inputs and masks.
+
+The two round differently, not more: the keeping pass rounds the scores, ALPHA and DATTN_DROP to 16 bits between its
+operators, the other one the unnormalised exponentials and the row sum's GAMMA.  Each is a relative error of half a unit
+(2^-11, bf16 2^-8) per tensor on the path, a handful of them in a row: 8 half-units is the bound used (GELU: no
+derivative jumps)."""
+
+import ctypes
+
+import pytest
+import torch
+
+from substation_b200 import Encoder, layouts as L, _lib
+from perf import cases
+
+pytestmark = pytest.mark.gpu
+HALF = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}
+
+
+def _passes(B, S, H, dtype, p, mode, lay, seed, activation='gelu'):
+    dev, E = torch.device('cuda:0'), 64 * H
+    table = L.validate(lay)
+    gen = torch.Generator(device=dev).manual_seed(seed)
+    sizes = L.sizes_map(B, S, H, E)
+    x0 = torch.randn(L.shape_of(table['X'], sizes), device=dev, generator=gen).to(dtype)
+    dy = torch.randn(x0.shape, device=dev, generator=gen).to(dtype)
+    masks = {n: (torch.rand(L.shape_of(table[n], sizes), device=dev, generator=gen) >= p).to(torch.uint8) for n in L.MASKS}
+    state, out = None, []
+    for keep in (True, False):
+        enc = Encoder('', B, S, H, E, lay, dtype, p, p, p, p, activation=activation, mask_mode=mode, seed=5,
+                      keep_all_intermediates=keep).to(dev)
+        with torch.no_grad():
+            if state is None:
+                for q in enc.params:
+                    q.copy_((torch.randn(q.shape, device=dev, generator=gen) * 0.1).to(dtype))
+                enc.S1.fill_(1)
+                enc.S2.fill_(1)
+                state = enc.state_dict()
+            else:
+                enc.load_state_dict(state)
+        if mode == 'explicit':
+            enc.set_masks(masks)
+        assert (enc.private_arena_bytes(dev) is None) == keep
+        x = x0.clone().requires_grad_(True)
+        y = enc(x)
+        y.backward(dy)
+        got = {'Y': y.detach(), 'DX': x.grad, **{n: q.grad for n, q in zip(enc._param_names, enc.params)}}
+        enc.philox_offset = 0
+        with torch.no_grad():                                # nothing is kept for a backward pass here
+            got['Y of inference'] = enc(x0)
+        out.append(got)
+        err = ctypes.c_int(0)
+        lib = _lib.load(_lib.dtype_key(dtype))
+        _lib.check(lib.sb_device_error(None, ctypes.byref(err)), lib)
+        assert err.value == 0
+    return out
+
+
+@pytest.mark.parametrize('B,S,H,dtype,p,mode,layouts', [
+    (1, 128, 2, torch.float16, 0.0, 'philox', 'uniform'),            # one tile, nothing dropped
+    (2, 16, 8, torch.float16, 0.1, 'philox', 'uniform'),             # rows shorter than a copy box
+    (3, 77, 4, torch.float16, 0.1, 'philox', 'uniform'),             # rows off the 16-byte grid: padded copies
+    (3, 77, 4, torch.float16, 0.1, 'explicit', 'uniform'),
+    (2, 130, 4, torch.float16, 0.1, 'explicit', 'uniform'),          # two columns in the second tile
+    (2, 136, 4, torch.bfloat16, 0.1, 'philox', 'uniform'),
+    (2, 512, 4, torch.float16, 0.1, 'explicit', 'uniform'),
+    (1, 1000, 2, torch.float16, 0.6, 'philox', 'uniform'),           # threshold with its top bit set, eight tiles
+    (40, 256, 4, torch.float16, 0.1, 'philox', 'uniform'),           # more items than a round of the machine
+    (160, 72, 2, torch.bfloat16, 0.1, 'philox', 'uniform'),
+    (5, 512, 8, torch.float16, 0.1, 'philox', 'feature_major'),      # activations change order on the way in and out
+    (3, 77, 4, torch.float16, 0.1, 'philox', 'feature_major'),
+    (2, 256, 4, torch.float16, 0.1, 'explicit', 'feature_major'),    # the caller's masks keep their order
+])
+def test_private_passes_match_passes_that_keep_everything(B, S, H, dtype, p, mode, layouts):
+    kept, private = _passes(B, S, H, dtype, p, mode, cases._layouts({'layouts': layouts}), seed=B * 1000 + S)
+    for name, want in kept.items():
+        got = private[name]
+        assert torch.isfinite(got).all(), name
+        err = ((got.double() - want.double()).norm() / want.double().norm()).item()
+        assert err <= 8 * HALF[dtype], (name, err)
+
+
+def test_private_passes_with_projections_stored_unit_by_unit():
+    """KKQQVV as QHBPJ (the order shipped for B=96, L=128 with the original module)."""
+    lay = L.uniform_layouts()
+    lay['forward_interm'] = [(n, 'QHBPJ' if n == 'KKQQVV' else d) for n, d in lay['forward_interm']]
+    kept, private = _passes(2, 256, 4, torch.float16, 0.1, 'philox', lay, seed=3)
+    for name, want in kept.items():
+        err = ((private[name].double() - want.double()).norm() / want.double().norm()).item()
+        assert err <= 8 * HALF[torch.float16], (name, err)
+
+
+def test_row_maxima_that_rise_by_more_than_the_lag():
+    """Scores that grow along the keys by far more than 2^8 per tile: every tile raises the reference maximum and
+    rescales what has been summed so far (std 1.5 projections, keys scaled up with their position)."""
+    dev, B, S, H = torch.device('cuda:0'), 2, 512, 2
+    E = 64 * H
+    enc = Encoder('', B, S, H, E, L.uniform_layouts(), torch.float16, 0., 0., 0., 0., activation='gelu').to(dev)
+    ref = Encoder('', B, S, H, E, L.uniform_layouts(), torch.float16, 0., 0., 0., 0., activation='gelu',
+                  keep_all_intermediates=True).to(dev)
+    gen = torch.Generator(device=dev).manual_seed(1)
+    with torch.no_grad():
+        for n, q in zip(enc._param_names, enc.params):
+            q.copy_((torch.randn(q.shape, device=dev, generator=gen) * (0.25 if n == 'WKQV' else 0.05)).half())
+        enc.S1.fill_(1)
+        enc.S2.fill_(1)
+    ref.load_state_dict(enc.state_dict())
+    x = torch.randn(B, S, E, device=dev, generator=gen) * torch.linspace(0.2, 3, S, device=dev)[None, :, None]
+    outs = []
+    for e in (ref, enc):
+        xi = x.half().requires_grad_(True)
+        y = e(xi)
+        y.backward(torch.ones_like(y) * torch.linspace(-1, 1, E, device=dev).half())
+        outs.append([y.detach(), xi.grad] + [q.grad for q in e.params])
+    for a, b in zip(*outs):
+        assert torch.isfinite(b).all()
+        # the keeping pass rounds scores of up to ~100 to 16 bits before exponentiating: errors of 2^-5 in ALPHA
+        assert ((a.double() - b.double()).norm() / a.double().norm()).item() <= 2.0 ** -5
