@@ -706,6 +706,9 @@ struct sb_encoder {
     void drop() { slot[0].drop(); slot[1].drop(); }
   };
   GraphCache graph_fwd, graph_bwd, graph_fwd_private, graph_bwd_private;
+  // The same layer with every intermediate in its logical order (parameters as configured): what private passes run
+  // when some activation of this configuration does not have its features innermost.
+  std::unique_ptr<sb_encoder> twin;
   bool rewriting = false;       // a pass is running that only rewrites a graph's kernel parameters
   cudaStream_t capture_stream = nullptr;
   cudaEvent_t ffn_grads_event = nullptr;   // recorded in backward once the feed-forward gradients are final
@@ -902,6 +905,30 @@ int einsum_fused(sb_encoder* e, cudaStream_t s, const char* name, Contract which
 
 }  // namespace
 
+namespace {
+
+// What a pass needs of the layouts, once they are known.
+void derive(sb_encoder* e) {
+  const auto& logical = logical_dims();
+  for (int i = 0; i < kTensors; ++i) e->dims[i] = e->layout.at(kTensorNames[i]);
+  for (int i = 0; i < kTensors; ++i)
+    e->logical[i] = e->view(nullptr, e->layout.at(kTensorNames[i]), logical.at(kTensorNames[i]));
+  e->proj = e->view(nullptr, e->layout["KKQQVV"].substr(1), "PHBJ");
+  e->dproj = e->view(nullptr, e->layout["DKKQQVV"].substr(1), "PHBJ");
+  e->contractions.resize(kContractions);
+}
+
+// Every activation has its features innermost: the case the elementwise and LayerNorm kernels have fast paths for.
+bool features_innermost(const sb_encoder* e) {
+  for (const auto& kv : logical_dims()) {
+    const std::string& l = kv.second;
+    if ((l == "BJI" || l == "BJU") && e->layout.at(kv.first).back() != l.back()) return false;
+  }
+  return true;
+}
+
+}  // namespace
+
 extern "C" int sb_encoder_create(const sb_encoder_config* cfg, sb_encoder** out) {
   if (!cfg || !out) return fail(SB_ERR_ARG, "sb_encoder_create: null argument");
   *out = nullptr;
@@ -949,12 +976,7 @@ extern "C" int sb_encoder_create(const sb_encoder_config* cfg, sb_encoder** out)
       return fail(SB_ERR_LAYOUT, std::string("sb_encoder_create: stacked tensor ") + n + " must have Q outermost");
   if (e->layout["X"] != e->layout["SB2"])
     return fail(SB_ERR_LAYOUT, "sb_encoder_create: input and output layouts must be equal so that layers chain");
-  for (int i = 0; i < kTensors; ++i) e->dims[i] = e->layout.at(kTensorNames[i]);
-  for (int i = 0; i < kTensors; ++i)
-    e->logical[i] = e->view(nullptr, e->layout.at(kTensorNames[i]), logical.at(kTensorNames[i]));
-  e->proj = e->view(nullptr, e->layout["KKQQVV"].substr(1), "PHBJ");
-  e->dproj = e->view(nullptr, e->layout["DKKQQVV"].substr(1), "PHBJ");
-  e->contractions.resize(kContractions);
+  derive(e.get());
   SB_CUDA_OK(cudaGetDevice(&e->device));
   // one allocation: token-reduction partials, then up to four fp32 partial copies of the largest weight gradient (the
   // stacked [3E, E] projection)
@@ -967,6 +989,19 @@ extern "C" int sb_encoder_create(const sb_encoder_config* cfg, sb_encoder** out)
     SB_CUDA_OK(cudaMalloc(&e->workspace, kWsBytes));
   }
   SB_CUDA_OK(cudaMemset(e->workspace, 0, kWsCounterBytes));   // the partial sums behind the counters need no value
+  if (!features_innermost(e.get())) {
+    e->twin.reset(new sb_encoder);
+    sb_encoder* t = e->twin.get();
+    t->B = e->B; t->S = e->S; t->H = e->H; t->I = e->I; t->P = e->P; t->U = e->U;
+    t->activation = e->activation;
+    t->p_softmax = e->p_softmax; t->p_resid1 = e->p_resid1; t->p_act = e->p_act; t->p_resid2 = e->p_resid2;
+    t->param_order = e->param_order; t->fwd_order = e->fwd_order; t->bwd_order = e->bwd_order;
+    t->layout = logical;
+    for (const char* n : kParamNames) t->layout[n] = e->layout.at(n);
+    t->workspace = e->workspace; t->gemm_ws = e->gemm_ws; t->gemm_ws_bytes = e->gemm_ws_bytes;   // owned by e
+    t->device = e->device;
+    derive(t);
+  }
   *out = e.release();
   return SB_OK;
 }
@@ -1579,26 +1614,63 @@ extern "C" int sb_encoder_backward(sb_encoder* e, void* stream, const void* dy, 
 
 namespace {
 
-int private_supported(const sb_encoder* e) {
+// The handle whose layouts a private pass of `e` uses.  Explicit masks are the caller's and keep their layouts.
+sb_encoder* private_target(sb_encoder* e, int mask_mode) {
+  if (!e->twin) return e;
+  if (mask_mode == SB_MASK_EXPLICIT)
+    for (int id : {TID("DROP1MASK"), TID("DROP2MASK"), TID("DROP3MASK")})
+      if (e->dims[id] != e->twin->dims[id]) return e;
+  return e->twin.get();
+}
+
+int private_supported(const sb_encoder* e, const sb_encoder* t) {
   if (e->dims[TID("ATTN_DROP_MASK")] != "HBJK" ||
-      flash_supported(e->H, e->B, e->S, e->P, proj_view(e->proj), proj_view(e->dproj), proj_view(e->logical[TID("GAMMA")]),
-                      proj_view(e->logical[TID("DGAMMA")])) != SB_OK)
+      flash_supported(e->H, e->B, e->S, e->P, proj_view(t->proj), proj_view(t->dproj), proj_view(t->logical[TID("GAMMA")]),
+                      proj_view(t->logical[TID("DGAMMA")])) != SB_OK)
     return fail(SB_ERR_UNSUPPORTED, "private passes need head size 64, score masks stored as HBJK and projections with unit "
                                     "stride along the head or the sequence dim");
   return SB_OK;
+}
+
+// Scratch of the attention kernels, then (for a twin of other activation layouts) two tensors of X's size.
+struct PrivateScratch { size_t attn_fwd, attn_bwd, act; };
+PrivateScratch private_scratch(const sb_encoder* e, const sb_encoder* t) {
+  FlashScratch f;
+  flash_scratch(e->H, e->B, e->S, flash_padded(proj_view(t->proj), e->S), flash_padded(proj_view(t->logical[TID("DGAMMA")]), e->S), &f);
+  const size_t act = t->dims[TID("X")] != e->dims[TID("X")] ? ((size_t)e->B * e->S * e->I * sizeof(sb_half) + 255) / 256 * 256 : 0;
+  return PrivateScratch{f.fwd_bytes, f.bwd_bytes, act};
+}
+
+// What a pass of the twin inherits from its handle, and hands back.
+void to_twin(sb_encoder* e, sb_encoder* t) {
+  if (t == e) return;
+  t->fuse = e->fuse; t->dead_stores = e->dead_stores;
+  t->ffn_grads_event = e->ffn_grads_event; t->rewriting = e->rewriting;
+}
+void from_twin(sb_encoder* e, const sb_encoder* t, long long kernels_before, bool forward) {
+  if (t == e) return;
+  e->launches = t->launches;
+  (forward ? e->kernels_fwd : e->kernels_bwd) = g_kernel_launches - kernels_before;
+}
+
+int relayout_x(sb_encoder* from, const void* src, sb_encoder* to, void* dst, cudaStream_t s) {
+  View3 a, b;
+  const sb_tensor ta = from->view(src, TID("X")), tb = to->view(dst, TID("X"));
+  SB_TRY(to_view3(&ta, nullptr, false, "relayout.src", &a));
+  SB_TRY(to_view3(&tb, &ta, false, "relayout.dst", &b));
+  return launch_relayout(s, dims3(&ta), a, b);
 }
 
 }  // namespace
 
 extern "C" int sb_encoder_private_bytes(sb_encoder* e, int mask_mode, size_t* forward, size_t* backward) {
   if (!e || !forward || !backward) return fail(SB_ERR_ARG, "sb_encoder_private_bytes: null argument");
-  (void)mask_mode;
   *forward = *backward = 0;
-  if (!e->fuse || e->dead_stores || private_supported(e) != SB_OK) return SB_OK;
-  FlashScratch f;
-  flash_scratch(e->H, e->B, e->S, flash_padded(proj_view(e->proj), e->S), flash_padded(proj_view(e->logical[TID("DGAMMA")]), e->S), &f);
-  *forward = f.fwd_bytes;
-  *backward = f.bwd_bytes;
+  const sb_encoder* t = private_target(e, mask_mode);
+  if (!e->fuse || e->dead_stores || private_supported(e, t) != SB_OK) return SB_OK;
+  const PrivateScratch p = private_scratch(e, t);
+  *forward = p.attn_fwd + 2 * p.act;
+  *backward = p.attn_bwd + 2 * p.act;
   return SB_OK;
 }
 
@@ -1607,9 +1679,20 @@ extern "C" int sb_encoder_forward_private(sb_encoder* e, void* stream, const voi
                                           uint64_t seed, uint64_t offset) {
   if (!e || !x || !y || !params || !fwd || !scratch) return fail(SB_ERR_ARG, "sb_encoder_forward_private: null argument");
   if (!aligned(scratch, 16)) return fail(SB_ERR_ALIGNMENT, "sb_encoder_forward_private: scratch is not 16-byte aligned");
-  SB_TRY(private_supported(e));
+  sb_encoder* t = private_target(e, mask_mode);
+  SB_TRY(private_supported(e, t));
+  const PrivateScratch ps = private_scratch(e, t);
+  char* acts = reinterpret_cast<char*>(scratch) + ps.attn_fwd;
   const PrivateForward priv{scratch, keep != 0};
-  auto pass = [&](cudaStream_t s) { return forward_pass(e, (void*)s, x, params, fwd, y, mask_mode, seed, offset, &priv); };
+  auto pass = [&](cudaStream_t s) {
+    const long long k0 = g_kernel_launches;
+    to_twin(e, t);
+    if (ps.act) SB_TRY(relayout_x(e, x, t, acts, s));
+    SB_TRY(forward_pass(t, (void*)s, ps.act ? acts : x, params, fwd, ps.act ? acts + ps.act : y, mask_mode, seed, offset, &priv));
+    if (ps.act) SB_TRY(relayout_x(t, acts + ps.act, e, y, s));
+    from_twin(e, t, k0, true);
+    return (int)SB_OK;
+  };
   return run_pass(e, e->graph_fwd_private, (cudaStream_t)stream, pass);
 }
 
@@ -1620,9 +1703,21 @@ extern "C" int sb_encoder_backward_private(sb_encoder* e, void* stream, const vo
     return fail(SB_ERR_ARG, "sb_encoder_backward_private: null argument");
   if (!aligned(fwd_scratch, 16) || !aligned(scratch, 16))
     return fail(SB_ERR_ALIGNMENT, "sb_encoder_backward_private: scratch is not 16-byte aligned");
-  (void)mask_mode;
-  SB_TRY(private_supported(e));
+  sb_encoder* t = private_target(e, mask_mode);
+  SB_TRY(private_supported(e, t));
+  const PrivateScratch ps = private_scratch(e, t);
+  const char* xt = reinterpret_cast<const char*>(fwd_scratch) + ps.attn_fwd;   // left there by the forward pass
+  char* acts = reinterpret_cast<char*>(scratch) + ps.attn_bwd;
   const PrivateBackward priv{fwd_scratch, scratch};
-  auto pass = [&](cudaStream_t s) { return backward_pass(e, (void*)s, dy, dparams, bwd, params, fwd, x, dx, &priv); };
+  auto pass = [&](cudaStream_t s) {
+    const long long k0 = g_kernel_launches;
+    to_twin(e, t);
+    if (ps.act) SB_TRY(relayout_x(e, dy, t, acts, s));
+    SB_TRY(backward_pass(t, (void*)s, ps.act ? acts : dy, dparams, bwd, params, fwd, ps.act ? xt : x,
+                         ps.act ? acts + ps.act : dx, &priv));
+    if (ps.act) SB_TRY(relayout_x(t, acts + ps.act, e, dx, s));
+    from_twin(e, t, k0, false);
+    return (int)SB_OK;
+  };
   return run_pass(e, e->graph_bwd_private, (cudaStream_t)stream, pass);
 }

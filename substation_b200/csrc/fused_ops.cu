@@ -1079,6 +1079,68 @@ int launch_bad(cudaStream_t s, Dims3 d, View3 in, const void* bias, View3 mask, 
   return SB_OK;
 }
 
+namespace {
+
+// Two orders of one tensor: 64 x 64 tiles over (rows, features) pass through shared memory, read along the source's
+// unit-stride dim and written along the destination's.  Rows are one of the two token dims, or both where they collapse
+// in both orders; the other one is `batch`.
+struct RelayoutParams {
+  const sb_half* src; long long s_row, s_f, s_batch;
+  sb_half* dst; long long d_row, d_f, d_batch;
+  int rows, F, tiles_r, tiles_f;
+  int src_rows, dst_rows;   // consecutive threads walk rows (else features)
+};
+__global__ void __launch_bounds__(256)
+relayout_kernel(const RelayoutParams p) {
+  __shared__ sb_half tile[64][66];
+  grid_dependency_sync();
+  const int tf = (int)(blockIdx.x % p.tiles_f), tr = (int)(blockIdx.x / p.tiles_f % p.tiles_r);
+  const long long b = blockIdx.x / ((long long)p.tiles_f * p.tiles_r);
+  const int x = threadIdx.x & 63, y = threadIdx.x >> 6;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int r = p.src_rows ? x : y + 4 * i, f = p.src_rows ? y + 4 * i : x;
+    if (tr * 64 + r < p.rows && tf * 64 + f < p.F)
+      tile[r][f] = p.src[b * p.s_batch + (tr * 64 + r) * p.s_row + (tf * 64 + f) * p.s_f];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int r = p.dst_rows ? x : y + 4 * i, f = p.dst_rows ? y + 4 * i : x;
+    if (tr * 64 + r < p.rows && tf * 64 + f < p.F)
+      p.dst[b * p.d_batch + (tr * 64 + r) * p.d_row + (tf * 64 + f) * p.d_f] = tile[r][f];
+  }
+}
+
+}  // namespace
+
+int launch_relayout(cudaStream_t s, Dims3 d, View3 src, View3 dst) {
+  if ((long long)d.B * d.J * d.F == 0) return SB_OK;
+  RelayoutParams p;
+  memset(&p, 0, sizeof(p));
+  p.src = reinterpret_cast<const sb_half*>(src.p);
+  p.dst = reinterpret_cast<sb_half*>(dst.p);
+  p.F = d.F;
+  p.s_f = src.sF; p.d_f = dst.sF;
+  long long batch;
+  if (src.sB == src.sJ * d.J && dst.sB == dst.sJ * d.J && (long long)d.B * d.J < 0x7fffffffLL) {
+    p.rows = d.B * d.J; p.s_row = src.sJ; p.d_row = dst.sJ;
+    batch = 1;
+  } else if (src.sB == 1 || dst.sB == 1) {
+    p.rows = d.B; p.s_row = src.sB; p.d_row = dst.sB; p.s_batch = src.sJ; p.d_batch = dst.sJ;
+    batch = d.J;
+  } else {
+    p.rows = d.J; p.s_row = src.sJ; p.d_row = dst.sJ; p.s_batch = src.sB; p.d_batch = dst.sB;
+    batch = d.B;
+  }
+  p.src_rows = src.sF != 1; p.dst_rows = dst.sF != 1;
+  p.tiles_r = (p.rows + 63) / 64; p.tiles_f = (d.F + 63) / 64;
+  const long long blocks = batch * p.tiles_r * p.tiles_f;
+  if (blocks > 0x7fffffffLL) return fail(SB_ERR_UNSUPPORTED, "relayout: too many tiles");
+  SB_LAUNCH_OK(launch_k(relayout_kernel, (unsigned)blocks, 256, 0, s, p));
+  return SB_OK;
+}
+
 int launch_bei(cudaStream_t s, Dims3 d, View3 a, View3 b, View3 out) {
   const long long R = (long long)d.B * d.J;
   if (R == 0 || d.F == 0) return SB_OK;

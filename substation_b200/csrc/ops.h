@@ -27,6 +27,8 @@ int launch_bad(cudaStream_t s, Dims3 d, View3 in, const void* bias, View3 mask, 
                View3 drop2, int activation, Rng rng);
 int launch_blnrd(cudaStream_t s, Dims3 d, View3 dln, View2 istd, View3 diff, View3 mask,
                  View3 dresid, View3 dlin);
+// dst = src, two orders of the same [B,J,F] tensor.
+int launch_relayout(cudaStream_t s, Dims3 d, View3 src, View3 dst);
 int launch_bei(cudaStream_t s, Dims3 d, View3 a, View3 b, View3 out);
 int launch_baib(cudaStream_t s, Dims5 d, View5 in, void* dbias, long long bsN, long long bsP,
                 long long bsH);
