@@ -391,11 +391,25 @@ __device__ __forceinline__ uint4 hadd8(const uint4& a, const uint4& b) {
   return o;
 }
 
+// Tanh-form GELU, x * (1 + tanh u) / 2 with u = 0.79788456 (x + 0.044715 x^3), written as x / (1 + 2^t) with
+// t = -2 u log2(e): (1 + tanh u) / 2 is the logistic function of 2u.  One ex2 and one rcp of the special-function unit
+// instead of tanhf's branches and division, and no cancellation where tanh u is close to -1 (at x = -4, 1 + tanhf(u) has
+// lost eleven bits).
+__device__ __forceinline__ float ex2_unit(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rcp_unit(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float gelu_exponent(float x) { return x * fmaf(x * x, -0.10294324f, -2.3022082f); }
+
 __device__ __forceinline__ float act_fwd(float x, int activation) {
   if (activation == SB_ACT_RELU) return fmaxf(x, 0.f);
-  // tanh-form GELU
-  const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
-  return 0.5f * x * (1.f + tanhf(u));
+  return x * rcp_unit(1.f + ex2_unit(gelu_exponent(x)));
 }
 
 // Contiguous per-feature vectors (bias, gamma, beta): [F], unit stride.
@@ -422,6 +436,27 @@ __device__ __forceinline__ void philox_keep8(const Rng& r, unsigned long long g,
   const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
   for (int t = 0; t < 8; ++t) m[t] = (((ww[t >> 1] >> (16 * (t & 1))) & 0xffffu) >= r.thr) ? 1u : 0u;
+}
+// The same eight flags as mask bytes.  The 16-bit lanes of a word are compared with the threshold together: with the top
+// bits forced on in the word and off in the threshold the subtraction cannot borrow across lanes, and word >= threshold
+// is the majority of the word's top bit, the threshold's inverted one and the difference's.
+__device__ __forceinline__ uint32_t sign_lanes(uint32_t v) {   // 0xffff in every 16-bit lane whose top bit is set
+  uint32_t d;
+  asm("prmt.b32 %0, %1, 0, 0xBB99;" : "=r"(d) : "r"(v));
+  return d;
+}
+__device__ __forceinline__ uint2 philox_mask8(const Rng& r, unsigned long long g) {
+  if (r.thr == 0u) return make_uint2(0x01010101u, 0x01010101u);   // nothing is dropped
+  const uint4 w = philox4x32_10(make_uint4((uint32_t)g, (uint32_t)(g >> 32), r.off_lo, r.off_hi), r.seed_lo, r.seed_hi);
+  const uint32_t thr2 = r.thr * 0x10001u, tl = thr2 & 0x7fff7fffu, nt = ~thr2;
+  const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+  uint32_t k[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t t = (ww[i] | 0x80008000u) - tl;
+    k[i] = sign_lanes((ww[i] & t) | (nt & (ww[i] | t)));
+  }
+  return make_uint2(__byte_perm(k[0], k[1], 0x6420) & 0x01010101u, __byte_perm(k[2], k[3], 0x6420) & 0x01010101u);
 }
 // Keep flags for eight consecutive logical indices e0..e0+7 that need not be group aligned.
 __device__ __forceinline__ void philox_keep8_unaligned(const Rng& r, unsigned long long e0,

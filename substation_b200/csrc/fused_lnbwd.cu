@@ -541,9 +541,7 @@ bdrln_ring_kernel(BdrlnParams p, int nstages, int stage_bytes) {
         if (mask_in) {
           mk = *reinterpret_cast<const uint2*>(st_m + (size_t)piece * 8);
         } else {
-          uint32_t mm[8];
-          philox_keep8(p.rng, ((unsigned long long)row * F + f) >> 3, mm);
-          mk = mask_pack(mm);
+          mk = philox_mask8(p.rng, ((unsigned long long)row * F + f) >> 3);
           store8m_raw(p.mask.p, off, 1, 1, f, F, mk);
         }
         float x[8], bb[8], rs[8];

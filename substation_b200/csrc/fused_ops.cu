@@ -36,11 +36,12 @@ __device__ __forceinline__ void philox8(const Rng& r, unsigned long long e0, uin
 
 __device__ __forceinline__ float act_bwd(float x, float dy, int activation) {
   if (activation == SB_ACT_RELU) return x > 0.f ? dy : 0.f;
-  const float x3 = x * x * x;
-  const float inner = 0.0356774f * x3 + 0.797885f * x;
-  const float th = tanhf(inner);
-  const float sech2 = 1.f - th * th;
-  return (0.5f * th + (0.0535161f * x3 + 0.398942f * x) * sech2 + 0.5f) * dy;
+  // d/dx of x * s(x) with s = 1 / (1 + q), q = 2^t as in act_fwd: s + x * s * (1 - s) * 2u', and 1 - s = q * s.
+  // (t is bounded so that q and s stay finite and normal.)
+  const float x2 = x * x;
+  const float q = ex2_unit(fminf(gelu_exponent(x), 126.f));
+  const float s = rcp_unit(1.f + q);
+  return s * fmaf(x * fmaf(x2, 0.21406448f, 1.5957691f), q * s, 1.f) * dy;
 }
 
 __device__ __forceinline__ uint4 hmul8(const uint4& a, const uint4& b) {
@@ -399,9 +400,7 @@ bad_flat_kernel(unsigned long long ngroups, int groups_per_row, const uint4* __r
       const unsigned long long g = g0 + u * stride;
       if (g >= ngroups) continue;
       if (rng.philox) {
-        uint32_t mm[8];
-        philox_keep8(rng, g, mm);
-        m[u] = mask_pack(mm);
+        m[u] = philox_mask8(rng, g);
         mask[g] = m[u];
       }
       const uint4 l = hadd8(x[u], bias[g % (unsigned)groups_per_row]);

@@ -322,11 +322,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
               // keep flags of the logical elements (m, nc + 8v ..): C is dense in logical order, so the
               // element index is the memory offset
 #pragma unroll
-              for (int v = 0; v < 8; ++v) {
-                uint32_t mm[8];
-                philox_keep8(p.epi.rng, (unsigned long long)(m * p.sCm + nc + 8 * v) >> 3, mm);
-                mk[v] = mask_pack(mm);
-              }
+              for (int v = 0; v < 8; ++v) mk[v] = philox_mask8(p.epi.rng, (unsigned long long)(m * p.sCm + nc + 8 * v) >> 3);
               if (row_ok) {
                 uint8_t* kp = p.epi.mask + m * p.sCm + nc;
 #pragma unroll
