@@ -278,12 +278,13 @@ extern "C" int sb_backward_softmax(void* stream, const sb_tensor* alpha, const s
   return launch_softmax_bwd((cudaStream_t)stream, dims4(alpha), va, vm, vg, vo);
 }
 
-extern "C" int sb_bias_dropout_residual_layernorm(void* stream, const sb_tensor* in, const sb_tensor* bias,
+// `keep` false: no backward pass follows, so what only that reads (DIFF, ISTD, LN, a generated mask) is not stored.
+static int bias_dropout_residual_layernorm(void* stream, const sb_tensor* in, const sb_tensor* bias,
                                                   const sb_tensor* resid, const sb_tensor* gamma,
                                                   const sb_tensor* beta, const sb_tensor* mask,
                                                   const sb_tensor* lin, const sb_tensor* diff,
                                                   const sb_tensor* istd, const sb_tensor* ln,
-                                                  const sb_tensor* out, const sb_dropout* dropout) {
+                                                  const sb_tensor* out, const sb_dropout* dropout, bool keep) {
   View3 vin, vres, vmask, vlin, vdiff, vln, vout;
   View2 vistd;
   void *pb, *pg, *pbt;
@@ -303,14 +304,28 @@ extern "C" int sb_bias_dropout_residual_layernorm(void* stream, const sb_tensor*
   SB_TRY(to_rng(dropout, &rng));
   if (lin && lin->ptr == in->ptr && (vlin.sB != vin.sB || vlin.sJ != vin.sJ || vlin.sF != vin.sF))
     return fail(SB_ERR_ARG, "bdrln: lin aliases in but has different strides");
+  if (!keep) {
+    vdiff.p = vln.p = vistd.p = nullptr;
+    if (rng.philox) vmask.p = nullptr;
+  }
   return launch_bdrln((cudaStream_t)stream, dims3(in), vin, pb, vres, pg, pbt, vmask, vlin, vdiff, vistd,
                       vln, vout, rng);
 }
 
-extern "C" int sb_bias_activation_dropout(void* stream, const sb_tensor* in, const sb_tensor* bias,
+extern "C" int sb_bias_dropout_residual_layernorm(void* stream, const sb_tensor* in, const sb_tensor* bias,
+                                                  const sb_tensor* resid, const sb_tensor* gamma,
+                                                  const sb_tensor* beta, const sb_tensor* mask,
+                                                  const sb_tensor* lin, const sb_tensor* diff,
+                                                  const sb_tensor* istd, const sb_tensor* ln,
+                                                  const sb_tensor* out, const sb_dropout* dropout) {
+  return bias_dropout_residual_layernorm(stream, in, bias, resid, gamma, beta, mask, lin, diff, istd, ln, out, dropout, true);
+}
+
+// `keep` as above: LIN1 and a generated mask are not stored when no backward pass follows.
+static int bias_activation_dropout(void* stream, const sb_tensor* in, const sb_tensor* bias,
                                           const sb_tensor* mask, const sb_tensor* lin1,
                                           const sb_tensor* drop2, int activation,
-                                          const sb_dropout* dropout) {
+                                          const sb_dropout* dropout, bool keep) {
   View3 vin, vmask, vlin, vdrop;
   void* pb;
   Rng rng;
@@ -321,7 +336,18 @@ extern "C" int sb_bias_activation_dropout(void* stream, const sb_tensor* in, con
   SB_TRY(to_view3(drop2, in, false, "bad.drop2", &vdrop));
   SB_TRY(to_param(bias, in->size[2], "bad.bias", &pb));
   SB_TRY(to_rng(dropout, &rng));
+  if (!keep) {
+    vlin.p = nullptr;
+    if (rng.philox) vmask.p = nullptr;
+  }
   return launch_bad((cudaStream_t)stream, dims3(in), vin, pb, vmask, vlin, vdrop, activation, rng);
+}
+
+extern "C" int sb_bias_activation_dropout(void* stream, const sb_tensor* in, const sb_tensor* bias,
+                                          const sb_tensor* mask, const sb_tensor* lin1,
+                                          const sb_tensor* drop2, int activation,
+                                          const sb_dropout* dropout) {
+  return bias_activation_dropout(stream, in, bias, mask, lin1, drop2, activation, dropout, true);
 }
 
 extern "C" int sb_backward_scale_bias(void* stream, void* workspace, const sb_tensor* dy, const sb_tensor* ln,
@@ -872,7 +898,7 @@ int einsum(sb_encoder* e, cudaStream_t s, const char* name, Contract which, cons
 // nothing marked) when the contraction kernel that can do it does not take this problem.
 template <class Dims>
 int einsum_fused(sb_encoder* e, cudaStream_t s, const char* name, Contract which, const void* a, const void* b, void* c,
-                 float alpha, const sb_epilogue* ep, const Dims& dims) {
+                 float alpha, const sb_epilogue* ep, const Dims& dims, bool keep = true) {
   sb_encoder::Contraction& k = e->contractions[which];
   const int mode = ep->dropout ? ep->dropout->mode : 0;   // in-kernel masks have conditions of their own
   if (k.status == -1 || k.mode != mode) {
@@ -894,6 +920,8 @@ int einsum_fused(sb_encoder* e, cudaStream_t s, const char* name, Contract which
   if (ep->out3) k.epi.out3 = ep->out3->ptr;
   if (ep->dropout) SB_TRY(to_rng(ep->dropout, &k.epi.rng));
   k.epi.skip_c = ep->discard_c ? 1 : 0;
+  k.epi.skip_out2 = keep ? 0 : 1;
+  if (!keep && ep->dropout && ep->dropout->mode == SB_MASK_PHILOX) k.epi.mask = nullptr;
   e->mark(s, name);
   const int st = run_einsum_fused(s, k.g, k.epi);
   if (st == SB_ERR_UNSUPPORTED || st == SB_ERR_ALIGNMENT) {
@@ -1148,6 +1176,7 @@ static int forward_pass(sb_encoder* e, void* stream, const void* x, const void* 
   auto lKK = [&] { return L(TID("KKQQVV")).substr(1); };
 
   auto v = [&](int id) { return e->view(T[id], id); };
+  const bool keep = !priv || priv->keep;   // a backward pass may follow
 
   // F1: stacked K,Q,V projections
   {
@@ -1230,8 +1259,8 @@ static int forward_pass(sb_encoder* e, void* stream, const void* x, const void* 
     sb_tensor istd = v(TID("LN1STD")), ln = v(TID("LN1")), out = v(TID("SB1"));
     sb_dropout d = drop(e->p_resid1, mask_mode, seed, offset + 1);
     // the biased projection is written back over ATT (nothing reads it again)
-    SB_TRY(sb_bias_dropout_residual_layernorm(stream, &in, &bias, &resid, &gamma, &beta, &mask,
-                                              e->dead_stores ? &in : nullptr, &diff, &istd, &ln, &out, &d));
+    SB_TRY(bias_dropout_residual_layernorm(stream, &in, &bias, &resid, &gamma, &beta, &mask,
+                                           e->dead_stores ? &in : nullptr, &diff, &istd, &ln, &out, &d, keep));
   }
   {
     // bias + activation + dropout in the epilogue of the first feed-forward contraction
@@ -1253,7 +1282,7 @@ static int forward_pass(sb_encoder* e, void* stream, const void* x, const void* 
       ep.logical_dims = "BJU";
       ep.discard_c = e->dead_stores ? 0 : 1;   // SB1_LINW1: only the bias operator reads it
       st = einsum_fused(e, s, "lin1+bad", kLin1Act, T[TID("SB1")], T[TID("LINW1")], T[TID("SB1_LINW1")], 1.f, &ep,
-                SB_DIMS(L(TID("SB1")), L(TID("LINW1")), lc));
+                SB_DIMS(L(TID("SB1")), L(TID("LINW1")), lc), keep);
       if (st != SB_OK && st != SB_ERR_UNSUPPORTED) return st;
     }
     if (st == SB_ERR_UNSUPPORTED) {
@@ -1263,7 +1292,7 @@ static int forward_pass(sb_encoder* e, void* stream, const void* x, const void* 
       sb_tensor in = v(TID("SB1_LINW1")), bias = v(TID("LINB1"));
       sb_tensor mask = v(TID("DROP2MASK")), lin1 = v(TID("LIN1"));
       sb_tensor d2 = v(TID("DROP2"));
-      SB_TRY(sb_bias_activation_dropout(stream, &in, &bias, &mask, &lin1, &d2, e->activation, &d));
+      SB_TRY(bias_activation_dropout(stream, &in, &bias, &mask, &lin1, &d2, e->activation, &d, keep));
     }
   }
   SB_TRY(einsum(e, s, "lin2", kLin2, T[TID("DROP2")], T[TID("LINW2")], T[TID("DROP2_LINW2")], 1.f,
@@ -1277,8 +1306,8 @@ static int forward_pass(sb_encoder* e, void* stream, const void* x, const void* 
     sb_tensor ln = v(TID("LN2")), out = v(TID("SB2"));
     sb_dropout d = drop(e->p_resid2, mask_mode, seed, offset + 3);
     // LIN2 is never read again
-    SB_TRY(sb_bias_dropout_residual_layernorm(stream, &in, &bias, &resid, &gamma, &beta, &mask,
-                                              e->dead_stores ? &lin : nullptr, &diff, &istd, &ln, &out, &d));
+    SB_TRY(bias_dropout_residual_layernorm(stream, &in, &bias, &resid, &gamma, &beta, &mask,
+                                           e->dead_stores ? &lin : nullptr, &diff, &istd, &ln, &out, &d, keep));
   }
   if (e->timing) { e->mark(s, ""); --e->launches; }
   e->kernels_fwd = g_kernel_launches - e->kernel_base;

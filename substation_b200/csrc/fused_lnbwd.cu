@@ -455,7 +455,7 @@ colsum_finish_kernel(const float* __restrict__ partial, int P, int F, int NQ, vo
 // four consecutive tokens, one bulk copy per tensor and block).  Warps 0-27 consume, one warp per token: block i of
 // the CTA lives in stage i % NS and belongs to the warp set i % 7 (warps 4 * set .. 4 * set + 3, one token each), so
 // the seven blocks a CTA gets at 4096 tokens on 148 SMs are one round (sixteen warps took two: 18.3 against 16.5 us).
-// Warp 28 produces.  A stage holds IN and RESID (4 x 2F bytes each) and, when the mask is an input, the mask rows
+// What only a backward pass reads (mask, DIFF, ISTD, LN) is not stored when its view is null.  Warp 28 produces.  A stage holds IN and RESID (4 x 2F bytes each) and, when the mask is an input, the mask rows
 // (4 x F bytes).  NV = 128-bit pieces per lane and row (F <= 256 * NV).
 // ---------------------------------------------------------------------------------------------------------
 constexpr int kFwdWarps = 28;
@@ -542,7 +542,7 @@ bdrln_ring_kernel(BdrlnParams p, int nstages, int stage_bytes) {
           mk = *reinterpret_cast<const uint2*>(st_m + (size_t)piece * 8);
         } else {
           mk = philox_mask8(p.rng, ((unsigned long long)row * F + f) >> 3);
-          store8m_raw(p.mask.p, off, 1, 1, f, F, mk);
+          if (p.mask.p) store8m_raw(p.mask.p, off, 1, 1, f, F, mk);
         }
         float x[8], bb[8], rs[8];
         unpack8(*reinterpret_cast<const uint4*>(st + (size_t)piece * 16), x);
@@ -576,7 +576,7 @@ bdrln_ring_kernel(BdrlnParams p, int nstages, int stage_bytes) {
       }
     }
     const float rstd = rsqrtf(warp_sum(sq) * invF + kLnEps);
-    if (lane == 0) reinterpret_cast<sb_half*>(p.istd.p)[b * p.istd.sB + j * p.istd.sJ] = sb_f2h(rstd);
+    if (lane == 0 && p.istd.p) reinterpret_cast<sb_half*>(p.istd.p)[b * p.istd.sB + j * p.istd.sJ] = sb_f2h(rstd);
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
       const int f = (lane + kWarp * k) * 8;
@@ -589,8 +589,8 @@ bdrln_ring_kernel(BdrlnParams p, int nstages, int stage_bytes) {
         n[e] = r[k][e] * rstd;
         o[e] = fmaf(n[e], gm[e], bt[e]);
       }
-      store8h_raw(p.diff.p, off, 1, 1, f, F, pack8(r[k]));
-      store8h_raw(p.ln.p, off, 1, 1, f, F, pack8(n));
+      if (p.diff.p) store8h_raw(p.diff.p, off, 1, 1, f, F, pack8(r[k]));
+      if (p.ln.p) store8h_raw(p.ln.p, off, 1, 1, f, F, pack8(n));
       store8h_raw(p.out.p, off, 1, 1, f, F, pack8(o));
     }
   }

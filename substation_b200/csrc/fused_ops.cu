@@ -253,7 +253,7 @@ bdrln_kernel(Dims3 d, View3 in, const void* bias, View3 resid, const void* gamma
           uint32_t mm[8];
           philox8<AV>(rng, (unsigned long long)row * d.F + f, mm);
           mr[i] = mask_pack(mm);
-          store8m_raw(mask.p, o_mask, mask.sF, SB_VEC(mask), f, d.F, mr[i]);
+          if (mask.p) store8m_raw(mask.p, o_mask, mask.sF, SB_VEC(mask), f, d.F, mr[i]);
         }
         const uint4 bs = load8h_raw(bias, 0, 1, AV || pvec, f, d.F);
         float x[8], bb[8], rs[8];
@@ -285,7 +285,7 @@ bdrln_kernel(Dims3 d, View3 in, const void* bias, View3 resid, const void* gamma
       }
     }
     const float rstd = rsqrtf(warp_sum(sq) * invF + kLnEps);
-    if (lane == 0) reinterpret_cast<sb_half*>(istd.p)[b * istd.sB + j * istd.sJ] = sb_f2h(rstd);
+    if (lane == 0 && istd.p) reinterpret_cast<sb_half*>(istd.p)[b * istd.sB + j * istd.sJ] = sb_f2h(rstd);
     const long long o_diff = b * diff.sB + j * diff.sJ, o_ln = b * ln.sB + j * ln.sJ;
     const long long o_out = b * out.sB + j * out.sJ;
 #pragma unroll
@@ -300,8 +300,8 @@ bdrln_kernel(Dims3 d, View3 in, const void* bias, View3 resid, const void* gamma
         n[e] = r[i][e] * rstd;
         o[e] = fmaf(n[e], gm[e], bt[e]);
       }
-      store8h_raw(diff.p, o_diff, diff.sF, SB_VEC(diff), f, d.F, pack8(r[i]));
-      store8h_raw(ln.p, o_ln, ln.sF, SB_VEC(ln), f, d.F, pack8(n));
+      if (diff.p) store8h_raw(diff.p, o_diff, diff.sF, SB_VEC(diff), f, d.F, pack8(r[i]));
+      if (ln.p) store8h_raw(ln.p, o_ln, ln.sF, SB_VEC(ln), f, d.F, pack8(n));
       store8h_raw(out.p, o_out, out.sF, SB_VEC(out), f, d.F, pack8(o));
     }
   }
@@ -401,10 +401,10 @@ bad_flat_kernel(unsigned long long ngroups, int groups_per_row, const uint4* __r
       if (g >= ngroups) continue;
       if (rng.philox) {
         m[u] = philox_mask8(rng, g);
-        mask[g] = m[u];
+        if (mask) mask[g] = m[u];
       }
       const uint4 l = hadd8(x[u], bias[g % (unsigned)groups_per_row]);
-      lin1[g] = l;
+      if (lin1) lin1[g] = l;
       uint4 a;
       if (ACT == SB_ACT_RELU) {
         const sb_half2* h = reinterpret_cast<const sb_half2*>(&l);
@@ -507,14 +507,14 @@ bad_kernel(Dims3 d, int spans, View3 in, const void* bias, View3 mask, View3 lin
     load8p(bias, f, d.F, AV || pvec, bs);
     if (rng.philox) {
       philox8<AV>(rng, (unsigned long long)row * d.F + f, m[i]);
-      store8m(mask.p, o_m, mask.sF, SB_VEC(mask), f, d.F, m[i]);
+      if (mask.p) store8m(mask.p, o_m, mask.sF, SB_VEC(mask), f, d.F, m[i]);
     }
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       x[i][e] += bs[e];
       o[e] = m[i][e] ? act_fwd(x[i][e], activation) : 0.f;
     }
-    store8h(lin1.p, o_l, lin1.sF, SB_VEC(lin1), f, d.F, x[i]);
+    if (lin1.p) store8h(lin1.p, o_l, lin1.sF, SB_VEC(lin1), f, d.F, x[i]);
     store8h(drop2.p, o_d, drop2.sF, SB_VEC(drop2), f, d.F, o);
   }
 }

@@ -257,6 +257,7 @@ struct EpiParams {
   uint8_t* mask;         // [M][N] bytes, row stride sCm; read, or written when rng.philox
   int activation;
   int skip_c;            // C itself is not stored (nothing reads it once the fused outputs exist)
+  int skip_out2;         // kind 3: the pre-activation and (mask == null) the generated mask are not stored either
   Rng rng;
 };
 
@@ -949,6 +950,7 @@ int launch_tc_pair(cudaStream_t s, const GemmProblem& g, const OperandMap& a, co
     p.epi.mask = reinterpret_cast<uint8_t*>(epi->mask);
     p.epi.activation = epi->activation;
     p.epi.skip_c = epi->skip_c;
+    p.epi.skip_out2 = epi->skip_out2;
     p.epi.rng = epi->rng;
   }
   const int kind = epi ? epi->kind : 0;

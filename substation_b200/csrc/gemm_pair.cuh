@@ -317,13 +317,13 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           if (EPI == 3) {
 #pragma unroll
             for (int v = 0; v < 8; ++v) o1[v] = hadd8(o1[v], side[v]);   // the biased pre-activation
-            put(&tmC2, o1);
+            if (!p.epi.skip_out2) put(&tmC2, o1);
             if (p.epi.rng.philox) {
               // keep flags of the logical elements (m, nc + 8v ..): C is dense in logical order, so the
               // element index is the memory offset
 #pragma unroll
               for (int v = 0; v < 8; ++v) mk[v] = philox_mask8(p.epi.rng, (unsigned long long)(m * p.sCm + nc + 8 * v) >> 3);
-              if (row_ok) {
+              if (row_ok && p.epi.mask) {
                 uint8_t* kp = p.epi.mask + m * p.sCm + nc;
 #pragma unroll
                 for (int v = 0; v < 4; ++v)

@@ -112,6 +112,7 @@ struct GemmEpilogue {
   void* out2;
   void* out3;
   int skip_c;          // do not store C itself (only the fused outputs are wanted)
+  int skip_out2;       // kind 3: do not store out2, nor (mask null) a generated mask
 };
 // The contraction with fused epilogue work; SB_ERR_UNSUPPORTED unless the problem runs on the paired-CTA
 // kernel with TMA stores (large, single batch, unit-stride columns, N a multiple of 64).
