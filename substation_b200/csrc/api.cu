@@ -1360,11 +1360,37 @@ static int backward_pass(sb_encoder* e, void* stream, const void* dy, void* cons
       return st;
     }
   }
-  SB_TRY(einsum(e, s, "dXlin2", kDxLin2, T[TID("DLIN2")], T[TID("LINW2")], T[TID("DDROP2")], 1.f,
-                SB_DIMS(L(TID("DLIN2")), L(TID("LINW2")), L(TID("DDROP2")))));
+  // dXlin2 with the dropout, the activation's derivative and LINB1's gradient in its epilogue when DDROP2 may stay unseen
+  int st_act = SB_ERR_UNSUPPORTED;
+  if (priv && e->fuse && L(TID("DDROP2")) == "BJU" && L(TID("LIN1")) == "BJU" && L(TID("DLIN1")) == "BJU" && L(TID("DROP2MASK")) == "BJU") {
+    sb_encoder::Contraction* k = nullptr;
+    SB_TRY(planned(e, kDxLin2, T[TID("DLIN2")], T[TID("LINW2")], T[TID("DDROP2")], 1.f,
+                   SB_DIMS(L(TID("DLIN2")), L(TID("LINW2")), L(TID("DDROP2"))), &k));
+    const long long rows = gemm_row_blocks((long long)e->B * e->S);
+    if (e->gemm_ws && (size_t)rows * e->U * sizeof(float) <= e->gemm_ws_bytes && k->g.M == (long long)e->B * e->S && k->g.sCn == 1) {
+      GemmEpilogue ep{};
+      ep.kind = 4;
+      ep.resid = T[TID("LIN1")];
+      ep.mask = T[TID("DROP2MASK")];
+      ep.activation = e->activation;
+      ep.out2 = T[TID("DLIN1")];
+      ep.partial = reinterpret_cast<float*>(e->gemm_ws);
+      e->mark(s, "dXlin2+bdrlb");
+      st_act = run_gemm_fused(s, k->g, ep);
+      if (st_act == SB_OK) {
+        SB_TRY(launch_colsum(s, ep.partial, (int)rows, e->U, D[TID("LINB1")]));
+      } else {
+        if (st_act != SB_ERR_UNSUPPORTED && st_act != SB_ERR_ALIGNMENT) return st_act;
+        e->unmark();
+      }
+    }
+  }
+  if (st_act != SB_OK)
+    SB_TRY(einsum(e, s, "dXlin2", kDxLin2, T[TID("DLIN2")], T[TID("LINW2")], T[TID("DDROP2")], 1.f,
+                  SB_DIMS(L(TID("DLIN2")), L(TID("LINW2")), L(TID("DDROP2")))));
   SB_TRY(einsum(e, s, "dWlin2", kDwLin2, T[TID("DLIN2")], T[TID("DROP2")], D[TID("LINW2")], 1.f,
                 SB_DIMS(L(TID("DLIN2")), L(TID("DROP2")), L(TID("LINW2")))));
-  {
+  if (st_act != SB_OK) {
     e->mark(s, "bdrlb");
     sb_tensor g = v(TID("DDROP2")), mask = v(TID("DROP2MASK")), lin1 = v(TID("LIN1")), o = v(TID("DLIN1")), db = dv(TID("LINB1"));
     SB_TRY(sb_backward_dropout_activation_bias(stream, ws, &g, &mask, &lin1, &o, &db, e->activation));

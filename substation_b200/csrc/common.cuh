@@ -412,6 +412,38 @@ __device__ __forceinline__ float act_fwd(float x, int activation) {
   return x * rcp_unit(1.f + ex2_unit(gelu_exponent(x)));
 }
 
+__device__ __forceinline__ float act_bwd(float x, float dy, int activation) {
+  if (activation == SB_ACT_RELU) return x > 0.f ? dy : 0.f;
+  // d/dx of x * s(x) with s = 1 / (1 + q), q = 2^t as in act_fwd: s + x * s * (1 - s) * 2u', and 1 - s = q * s.
+  // (t is bounded so that q and s stay finite and normal.)
+  const float x2 = x * x;
+  const float q = ex2_unit(fminf(gelu_exponent(x), 126.f));
+  const float s = rcp_unit(1.f + q);
+  return s * fmaf(x * fmaf(x2, 0.21406448f, 1.5957691f), q * s, 1.f) * dy;
+}
+
+// Dropout and activation backward of eight packed values: act'(x) * mask * g (ReLU: exact selections of 16-bit values).
+__device__ __forceinline__ uint4 act_bwd8(const uint4& g, const uint4& x, const uint2& m, int activation) {
+  uint4 out;
+  if (activation == SB_ACT_RELU) {
+    const uint4 gm = mask_apply(g, m);
+    const sb_half2* xx = reinterpret_cast<const sb_half2*>(&x);
+    const sb_half2* gg = reinterpret_cast<const sb_half2*>(&gm);
+    sb_half2* q = reinterpret_cast<sb_half2*>(&out);
+    const sb_half2 zero = sb_f2h2_dup(0.f);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) q[i] = __hmul2(gg[i], __hgt2(xx[i], zero));
+  } else {
+    float gf[8], xf[8], o[8];
+    unpack8(g, gf);
+    unpack8(x, xf);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) o[e] = act_bwd(xf[e], mask_keep(m, e) ? gf[e] : 0.f, activation);
+    out = pack8(o);
+  }
+  return out;
+}
+
 // Contiguous per-feature vectors (bias, gamma, beta): [F], unit stride.
 __device__ __forceinline__ void load8p(const void* base, int f, int F, int vec, float v[8]) {
   load8h(base, 0, 1, vec, f, F, v, 0.f);

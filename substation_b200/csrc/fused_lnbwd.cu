@@ -419,7 +419,7 @@ lnbwd_ring_kernel(LnBwdParams p, int nstages, int stage_bytes) {
 // issued eight at a time, then added in row order) and are combined through shared memory in group order.
 constexpr int kFinishParts = 16;
 __global__ void __launch_bounds__(64 * kFinishParts)
-colsum_finish_kernel(const float* __restrict__ partial, int P, int F, int NQ, void* o0, void* o1, void* o2, void* o3) {
+colsum_finish_kernel(const float* __restrict__ partial, int P, int F, int ld, void* o0, void* o1, void* o2, void* o3) {
   grid_dependency_sync();
   __shared__ float sm[kFinishParts][64];
   const int q = blockIdx.y;
@@ -427,13 +427,13 @@ colsum_finish_kernel(const float* __restrict__ partial, int P, int F, int NQ, vo
   const int f = blockIdx.x * 64 + fl;
   float v = 0.f;
   if (f < F) {
-    const float* base = partial + (long long)q * P * kMaxF + f;
+    const float* base = partial + (long long)q * P * ld + f;
     for (int c0 = part; c0 < P; c0 += 8 * kFinishParts) {
       float x[8];
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         const int c = c0 + u * kFinishParts;
-        x[u] = c < P ? __ldcg(base + (long long)c * kMaxF) : 0.f;
+        x[u] = c < P ? __ldcg(base + (long long)c * ld) : 0.f;
       }
 #pragma unroll
       for (int u = 0; u < 8; ++u) v += x[u];
@@ -655,12 +655,17 @@ int launch(cudaStream_t s, void* ws, const LnBwdParams& p0, void* const outs[4])
   }
   SB_CUDA_OK(cudaGetLastError());
   dim3 grid((p.d.F + 63) / 64, NQ);
-  SB_LAUNCH_OK(launch_k(colsum_finish_kernel, grid, 64 * kFinishParts, 0, s, p.partial, P, p.d.F, NQ, outs[0], outs[1], outs[2], outs[3]));
+  SB_LAUNCH_OK(launch_k(colsum_finish_kernel, grid, 64 * kFinishParts, 0, s, p.partial, P, p.d.F, kMaxF, outs[0], outs[1], outs[2], outs[3]));
   SB_CUDA_OK(cudaGetLastError());
   return SB_OK;
 }
 
 }  // namespace
+
+int launch_colsum(cudaStream_t s, const float* partial, int P, int F, void* out) {
+  SB_LAUNCH_OK(launch_k(colsum_finish_kernel, dim3((F + 63) / 64, 1), 64 * kFinishParts, 0, s, partial, P, F, F, out, nullptr, nullptr, nullptr));
+  return SB_OK;
+}
 
 int launch_lnbwd_a(cudaStream_t s, void* ws, Dims3 d, View3 dy, View3 ln, const void* gamma, View2 istd, View3 diff,
                    View3 mask, View3 dln, View3 dresid, View3 dlin, void* dgamma, void* dbeta) {

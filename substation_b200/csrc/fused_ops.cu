@@ -34,16 +34,6 @@ __device__ __forceinline__ void philox8(const Rng& r, unsigned long long e0, uin
   else philox_keep8_unaligned(r, e0, m);
 }
 
-__device__ __forceinline__ float act_bwd(float x, float dy, int activation) {
-  if (activation == SB_ACT_RELU) return x > 0.f ? dy : 0.f;
-  // d/dx of x * s(x) with s = 1 / (1 + q), q = 2^t as in act_fwd: s + x * s * (1 - s) * 2u', and 1 - s = q * s.
-  // (t is bounded so that q and s stay finite and normal.)
-  const float x2 = x * x;
-  const float q = ex2_unit(fminf(gelu_exponent(x), 126.f));
-  const float s = rcp_unit(1.f + q);
-  return s * fmaf(x * fmaf(x2, 0.21406448f, 1.5957691f), q * s, 1.f) * dy;
-}
-
 __device__ __forceinline__ uint4 hmul8(const uint4& a, const uint4& b) {
   uint4 o;
   const sb_half2* x = reinterpret_cast<const sb_half2*>(&a);
@@ -742,26 +732,9 @@ struct BdrlbOp {
   template <bool AV>
   __device__ __forceinline__ void finish(int b, int j, int f, int F, const uint4&,
                                          const RowRegs<NIN>& r, float acc[NQ][8]) const {
-    uint4 out;
+    const uint4 out = act_bwd8(r.v[0], r.v[1], r.m, activation);
     float o[8];
-    if (activation == SB_ACT_RELU) {
-      // dlin1 = [lin1 > 0] * mask * ddrop2, all exact selections of fp16 values
-      const uint4 g = mask_apply(r.v[0], r.m);
-      const sb_half2* x = reinterpret_cast<const sb_half2*>(&r.v[1]);
-      const sb_half2* gg = reinterpret_cast<const sb_half2*>(&g);
-      sb_half2* q = reinterpret_cast<sb_half2*>(&out);
-      const sb_half2 zero = sb_f2h2_dup(0.f);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) q[i] = __hmul2(gg[i], __hgt2(x[i], zero));
-      unpack8(out, o);
-    } else {
-      float g[8], x[8];
-      unpack8(r.v[0], g);
-      unpack8(r.v[1], x);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) o[e] = act_bwd(x[e], mask_keep(r.m, e) ? g[e] : 0.f, activation);
-      out = pack8(o);
-    }
+    unpack8(out, o);
 #pragma unroll
     for (int e = 0; e < 8; ++e) acc[0][e] += (AV || f + e < F) ? o[e] : 0.f;
     store8h_raw(dlin1.p, b * dlin1.sB + j * dlin1.sJ, dlin1.sF, SB_VEC(dlin1), f, F, out);

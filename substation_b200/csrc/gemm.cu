@@ -249,6 +249,8 @@ __device__ int g_tc_error = 0;  // first failure code of any tcgen05 kernel on t
 //   kind 1: out2 = C + bias                        (attention input biases)
 //   kind 2: out2 = C + resid                       (encoder-input gradient)
 //   kind 3: out2 = C + bias, out3 = mask * act(out2)   (bias + activation + dropout)
+//   kind 4: out2 = act'(resid) * mask * C, and its column sums per 32 rows   (dropout + activation backward, bias
+//           gradient); C itself is never stored
 struct EpiParams {
   int kind;
   int vec_along_m;       // bias indexed by the row (m) instead of the column (n)
@@ -259,6 +261,7 @@ struct EpiParams {
   int skip_c;            // C itself is not stored (nothing reads it once the fused outputs exist)
   int skip_out2;         // kind 3: the pre-activation and (mask == null) the generated mask are not stored either
   Rng rng;
+  float* partial;        // kind 4: column sums, one row of N floats per 32 rows of C
 };
 
 struct TcParams {
@@ -941,9 +944,9 @@ int launch_tc_pair(cudaStream_t s, const GemmProblem& g, const OperandMap& a, co
     auto misaligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) != 0; };
     if ((epi->kind == 1 || epi->kind == 3) && !p.epi.vec_along_m && misaligned(epi->vec))
       return fail(SB_ERR_ALIGNMENT, "fused epilogue: a bias along the columns must be 16-byte aligned");
-    if (epi->kind == 2 && misaligned(epi->resid))
+    if ((epi->kind == 2 || epi->kind == 4) && misaligned(epi->resid))
       return fail(SB_ERR_ALIGNMENT, "fused epilogue: the residual must be 16-byte aligned");
-    if (epi->kind == 3 && (misaligned(epi->mask) || g.sCm % 16 != 0))
+    if ((epi->kind == 3 || epi->kind == 4) && (misaligned(epi->mask) || g.sCm % 16 != 0))
       return fail(SB_ERR_ALIGNMENT, "fused epilogue: the mask must be 16-byte aligned with a row pitch that is a multiple of 16");
     p.epi.vec = reinterpret_cast<const sb_half*>(epi->vec);
     p.epi.resid = reinterpret_cast<const sb_half*>(epi->resid);
@@ -952,6 +955,7 @@ int launch_tc_pair(cudaStream_t s, const GemmProblem& g, const OperandMap& a, co
     p.epi.skip_c = epi->skip_c;
     p.epi.skip_out2 = epi->skip_out2;
     p.epi.rng = epi->rng;
+    p.epi.partial = epi->partial;
   }
   const int kind = epi ? epi->kind : 0;
   auto launch = [&](auto kernel, int threads, int smem) {
@@ -960,13 +964,13 @@ int launch_tc_pair(cudaStream_t s, const GemmProblem& g, const OperandMap& a, co
     if (ea != cudaSuccess) return ea;
     return launch_k(kernel, 2 * nclusters, threads, smem, s, a.map, b.map, cmap, cmap2, cmap3, p);
   };
-  if (kind < 0 || kind > 3) return fail(SB_ERR_ARG, "fused epilogue: unknown kind");
+  if (kind < 0 || kind > 4) return fail(SB_ERR_ARG, "fused epilogue: unknown kind");
 #define SB_PAIR_CASE(K, EW)                                                                             \
   if (kind == K && ew == EW)                                                                            \
     SB_LAUNCH_OK(launch(pair::gemm_tc_pair_kernel<K, EW>, pair::Cfg<EW>::kThreads, pair::Cfg<EW>::kSmemBytes))
   const int ew = pair_epi_warps();
-  SB_PAIR_CASE(0, 4); SB_PAIR_CASE(1, 4); SB_PAIR_CASE(2, 4); SB_PAIR_CASE(3, 4);
-  SB_PAIR_CASE(0, 8); SB_PAIR_CASE(1, 8); SB_PAIR_CASE(2, 8); SB_PAIR_CASE(3, 8);
+  SB_PAIR_CASE(0, 4); SB_PAIR_CASE(1, 4); SB_PAIR_CASE(2, 4); SB_PAIR_CASE(3, 4); SB_PAIR_CASE(4, 4);
+  SB_PAIR_CASE(0, 8); SB_PAIR_CASE(1, 8); SB_PAIR_CASE(2, 8); SB_PAIR_CASE(3, 8); SB_PAIR_CASE(4, 8);
 #undef SB_PAIR_CASE
   SB_CUDA_OK(cudaGetLastError());
   return SB_OK;
@@ -1081,7 +1085,8 @@ int launch_gemm_tcgen05_epi(cudaStream_t s, const GemmProblem& g0, void* ws, siz
   // (ties: keep N as the unit-stride index of C so rows are stored as full lines).
   GemmProblem g = g0;
   const long long w0 = padded_work(g.M, g.N), w1 = padded_work(g.N, g.M);
-  const bool swap = (w1 < w0) || (w1 == w0 && g.sCn != 1 && g.sCm == 1);
+  // With fused epilogue work the rows of C have to be the stored lines.
+  const bool swap = epi ? g.sCn != 1 && g.sCm == 1 : (w1 < w0) || (w1 == w0 && g.sCn != 1 && g.sCm == 1);
   if (swap) {
     std::swap(g.M, g.N);
     std::swap(g.A, g.B);

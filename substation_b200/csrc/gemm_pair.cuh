@@ -286,12 +286,16 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
               for (int v = 0; v < 8; ++v) side[v] = *reinterpret_cast<const uint4*>(p.epi.vec + nc + 8 * v);
             }
           }
-          if (EPI == 2 && row_ok) {
+          if (EPI == 4) {
+#pragma unroll
+            for (int v = 0; v < 8; ++v) { side[v] = make_uint4(0, 0, 0, 0); mk[v] = make_uint2(0, 0); }
+          }
+          if ((EPI == 2 || EPI == 4) && row_ok) {
             const sb_half* rp = p.epi.resid + m * p.sCm + nc;
 #pragma unroll
             for (int v = 0; v < 8; ++v) side[v] = *reinterpret_cast<const uint4*>(rp + 8 * v);
           }
-          if (EPI == 3 && !p.epi.rng.philox && row_ok) {
+          if ((EPI == 4 || (EPI == 3 && !p.epi.rng.philox)) && row_ok) {
             const uint8_t* kp = p.epi.mask + m * p.sCm + nc;
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
@@ -308,11 +312,26 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[v * 8 + e]) * p.alpha;
             o1[v] = pack8(f);
           }
-          if (EPI == 0 || !p.epi.skip_c) put(&tmC, o1);
+          if (EPI == 0 || (EPI != 4 && !p.epi.skip_c)) put(&tmC, o1);
           if (EPI == 1 || EPI == 2) {
 #pragma unroll
             for (int v = 0; v < 8; ++v) o1[v] = hadd8(o1[v], side[v]);
             put(&tmC2, o1);
+          }
+          if (EPI == 4) {
+#pragma unroll
+            for (int v = 0; v < 8; ++v) o1[v] = act_bwd8(o1[v], side[v], mk[v], p.epi.activation);
+            put(&tmC2, o1);
+            // column sums of the 32 x 64 block from its staging rows: lane = two columns, no bank conflicts
+            const uint8_t* st = my_stage_gen + ((nstore - 1u) & 1u) * 4096;
+            float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              const float2 f = sb_h22f2(*reinterpret_cast<const sb_half2*>(st + i * 128 + (((lane >> 2) ^ (i & 7)) << 4) + (lane & 3) * 4));
+              s0 += f.x;
+              s1 += f.y;
+            }
+            if (nc < p.N) *reinterpret_cast<float2*>(p.epi.partial + (long long)(mc >> 5) * p.N + nc + 2 * lane) = make_float2(s0, s1);
           }
           if (EPI == 3) {
 #pragma unroll

@@ -49,6 +49,9 @@ int launch_lnbwd_b(cudaStream_t s, void* ws, Dims3 d, View3 ln1, const void* gam
                    View3 dlin2, View2 istd, View3 diff, View3 mask, View3 dln1, View3 dresid1, View3 datt,
                    void* dgamma1, void* dbeta1, void* dlinb2, void* dbo);
 
+// out[f] = sum of P partial rows of F floats, in a fixed order.
+int launch_colsum(cudaStream_t s, const float* partial, int P, int F, void* out);
+
 // bias + dropout + residual + LayerNorm with the input rows staged through a shared-memory ring (bulk copies);
 // SB_ERR_UNSUPPORTED, nothing launched, unless every view is feature-innermost with 16-byte-multiple rows.
 int launch_bdrln_ring(cudaStream_t s, Dims3 d, View3 in, const void* bias, View3 resid, const void* gamma,
@@ -102,7 +105,8 @@ struct GemmProblem {
 // Elementwise work fused behind the epilogue of a contraction (see EpiParams in gemm.cu).  out2 / out3 / resid /
 // mask have C's shape and strides (mask: in bytes); vec is a dense vector over C's rows (vec_along_m) or columns.
 struct GemmEpilogue {
-  int kind;            // 1 bias -> out2; 2 residual -> out2; 3 bias + activation + dropout -> out2, out3
+  int kind;            // 1 bias -> out2; 2 residual -> out2; 3 bias + activation + dropout -> out2, out3;
+                       // 4 dropout and activation backward at pre-activation `resid` -> out2, column sums -> partial
   int vec_along_m;
   const void* vec;
   const void* resid;
@@ -112,11 +116,13 @@ struct GemmEpilogue {
   void* out2;
   void* out3;
   int skip_c;          // do not store C itself (only the fused outputs are wanted)
+  float* partial;      // kind 4: [gemm_row_blocks(M)][N] column sums of out2 over blocks of 32 rows
   int skip_out2;       // kind 3: do not store out2, nor (mask null) a generated mask
 };
 // The contraction with fused epilogue work; SB_ERR_UNSUPPORTED unless the problem runs on the paired-CTA
 // kernel with TMA stores (large, single batch, unit-stride columns, N a multiple of 64).
 int run_gemm_fused(cudaStream_t s, const GemmProblem& g, const GemmEpilogue& epi);
+inline long long gemm_row_blocks(long long M) { return (M + 255) / 256 * 8; }
 
 // Collapse an einsum over strided operands into one batched GEMM (error if it is not one).
 int plan_einsum(const char* a_dims, const sb_tensor* a, const char* b_dims, const sb_tensor* b,
