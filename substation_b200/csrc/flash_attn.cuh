@@ -500,7 +500,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const uint32_t slots = (raw + 1023u) & ~1023u;
   const uint32_t sds = slots + kSlots * 2 * kTile, spm = sds + 2 * kTile, bars = spm + 2 * kTile;
   const uint32_t full = bars, empty = full + 8 * kSlots, sd_full = empty + 8 * kSlots, sd_empty = sd_full + 8;
-  const uint32_t pd_full = sd_empty + 8, pd_empty = pd_full + 8, acc_full = pd_empty + 8, acc_empty = acc_full + 16;
+  const uint32_t pd_full = sd_empty + 8, ds_empty = pd_full + 8, acc_full = ds_empty + 16, acc_empty = acc_full + 16;
   uint8_t* gen = smem_raw + (slots - raw);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen + (acc_empty + 16 - slots));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -515,8 +515,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     mbar_init(sd_full, 1);
     mbar_init(sd_empty, 8);
     mbar_init(pd_full, 8);
-    mbar_init(pd_empty, 1);
     for (int i = 0; i < 2; ++i) {
+      mbar_init(ds_empty + 8 * i, 1);
       mbar_init(acc_full + 8 * i, 1);
       mbar_init(acc_empty + 8 * i, 8);
     }
@@ -575,8 +575,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     SlotQueue sq;
     uint32_t phase = 0, n = 0, it = 0;
     bool ok = true;
-    struct Pending { int item, held, slot; uint32_t it; bool first, last; };
-    Pending pend{-1, 0, 0, 0u, false, false};
+    struct Pending { int item, held, slot; uint32_t it, n; bool first, last; };
+    Pending pend{-1, 0, 0, 0u, 0u, false, false};
     uint32_t npd = 0;
     auto wait_slot = [&](int s) {
       ok = __all_sync(0xffffffffu, mbar_wait(full + 8 * s, (phase >> s) & 1u, 32)) && ok;
@@ -596,12 +596,13 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         const uint32_t acc = tmem_acc + set * 128u;
         if (!qi) {
           mma_outputs(acc, spm, qt + kTile, p.g_jc, true, !d.first);          // dV += (mask * ALPHA)^T DGAMMA
+          umma_commit(ds_empty + 8);
           mma_outputs(acc + 64u, sds, qt, p.jc, true, !d.first);              // dK += DBETA^T Q
           if (p.both) mma_outputs(acc + 128u, sds, kt, p.jc, false, false);   // dQ  = DBETA K
         } else {
-          mma_outputs(acc, sds, kt, p.jc, false, !d.first);                   // dQ += DBETA K
+          mma_outputs(acc, d.n & 1u ? spm : sds, kt, p.jc, false, !d.first);  // dQ += DBETA K
         }
-        umma_commit(pd_empty);
+        umma_commit(qi && (d.n & 1u) ? ds_empty + 8 : ds_empty);
         umma_commit(empty + 8 * d.slot);
         if (d.last) {
           umma_commit(empty + 8 * d.held);
@@ -629,7 +630,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         }
         __syncwarp();
         if (pend.item >= 0) outputs(pend);
-        pend = Pending{item, held, s, it, t == 0, t == nb - 1};
+        pend = Pending{item, held, s, it, n, t == 0, t == nb - 1};
       }
     }
     if (ok && pend.item >= 0) outputs(pend);
@@ -668,9 +669,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // row inputs of a tile, asked for one tile ahead
     float lse = INFINITY, ds = 0.f;
     uint2 keep = make_uint2(0u, 0u);
-    auto fetch = [&](int item, int t) {
-      const bool qi = is_q(item);
-      const int u = unit_of(item), b = block_of(item);
+    auto fetch = [&](bool qi, int u, int b, int t) {
       const int j = (qi ? b : t) * 128 + rt, kb = qi ? t : b;
       lse = INFINITY; ds = 0.f;
       keep = make_uint2(0u, 0u);
@@ -680,11 +679,27 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         keep = reinterpret_cast<const uint2*>(p.bits + ((long long)u * nb + kb) * L + j)[h];
       }
     };
-    if ((int)blockIdx.x < p.items) fetch(blockIdx.x, 0);
+    // the two 16-bit tiles of shared memory: dK/dV items fill DBETA (0) and mask * ALPHA (1), dQ items alternate between
+    // them; `fills` counts the uses of each, and a tile is free once the products that read its last use are done
+    uint32_t fills0 = 0, fills1 = 0;
+    auto wait_tile = [&](int i) {
+      uint32_t& f = i ? fills1 : fills0;
+      if (f > 0) ok = __all_sync(0xffffffffu, mbar_wait(ds_empty + 8 * i, (f - 1u) & 1u, 38));
+      ++f;
+      return ok;
+    };
+    bool qi = false, next_qi = false;
+    int u = 0, b = 0, next_u = 0, next_b = 0;
+    if ((int)blockIdx.x < p.items) {
+      next_qi = is_q(blockIdx.x); next_u = unit_of(blockIdx.x); next_b = block_of(blockIdx.x);
+      fetch(next_qi, next_u, next_b, 0);
+    }
     int prev = -1;
     for (int item = blockIdx.x; item < p.items && ok; item += gridDim.x, ++it) {
-      const bool qi = is_q(item);
-      const int b = block_of(item);
+      qi = next_qi; u = next_u; b = next_b;
+      const int next = item + (int)gridDim.x;
+      const bool more = next < p.items;
+      if (more) { next_qi = is_q(next); next_u = unit_of(next); next_b = block_of(next); }
       for (int t = 0; t < nb && ok; ++t, ++n) {
         const int rem = L - (qi ? t : b) * 128 - h * 64;
         ok = __all_sync(0xffffffffu, mbar_wait(sd_full, n & 1u, 37));
@@ -720,18 +735,20 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             db[c * 16 + i] = pack2(fmaf(m0, __uint_as_float(rg[2 * i]), -ds * a0), fmaf(m1, __uint_as_float(rg[2 * i + 1]), -ds * a1));
           }
         }
-        if (t + 1 < nb) fetch(item, t + 1);
-        else if (item + (int)gridDim.x < p.items) fetch(item + gridDim.x, 0);
-        if (n > 0) {
-          ok = __all_sync(0xffffffffu, mbar_wait(pd_empty, (n - 1u) & 1u, 38));
-          if (!ok) break;
-        }
+        if (t + 1 < nb) fetch(qi, u, b, t + 1);
+        else if (more) fetch(next_qi, next_u, next_b, 0);
+        if (!qi) {
+          if (!wait_tile(1)) break;
 #pragma unroll
-        for (int v = 0; v < 8; ++v) {
-          const int o = (v ^ (lane & 7)) << 4;
-          *reinterpret_cast<uint4*>(drow + o) = make_uint4(db[4 * v], db[4 * v + 1], db[4 * v + 2], db[4 * v + 3]);
-          if (!qi) *reinterpret_cast<uint4*>(prow + o) = make_uint4(pm[4 * v], pm[4 * v + 1], pm[4 * v + 2], pm[4 * v + 3]);
+          for (int v = 0; v < 8; ++v)
+            *reinterpret_cast<uint4*>(prow + ((v ^ (lane & 7)) << 4)) = make_uint4(pm[4 * v], pm[4 * v + 1], pm[4 * v + 2], pm[4 * v + 3]);
         }
+        const bool alt = qi && (n & 1u);
+        if (!wait_tile(alt ? 1 : 0)) break;
+        uint8_t* dst = alt ? prow : drow;
+#pragma unroll
+        for (int v = 0; v < 8; ++v)
+          *reinterpret_cast<uint4*>(dst + ((v ^ (lane & 7)) << 4)) = make_uint4(db[4 * v], db[4 * v + 1], db[4 * v + 2], db[4 * v + 3]);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(pd_full);
