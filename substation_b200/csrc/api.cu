@@ -733,8 +733,9 @@ struct sb_encoder {
   };
   GraphCache graph_fwd, graph_bwd, graph_fwd_private, graph_bwd_private;
   // The same layer with every intermediate in its logical order (parameters as configured): what private passes run
-  // when some activation of this configuration does not have its features innermost.
+  // when some activation of this configuration does not have its features innermost, or the token count is off the 8 grid.
   std::unique_ptr<sb_encoder> twin;
+  bool private_pass = false;    // the pass running is a private one
   bool rewriting = false;       // a pass is running that only rewrites a graph's kernel parameters
   cudaStream_t capture_stream = nullptr;
   cudaEvent_t ffn_grads_event = nullptr;   // recorded in backward once the feed-forward gradients are final
@@ -763,6 +764,10 @@ struct sb_encoder {
     for (char c : dims) n *= extent(c);
     return n;
   }
+  // Tokens between two rows of a head-first tensor (..HBJ) when they are not B * S: a private pass over a token count off
+  // the 8 grid pads those rows to it, or no tensor map could address them.
+  long long token_pitch = 0;
+  long long slice() const { return (long long)P * H * (token_pitch ? token_pitch : (long long)B * S); }
   // Tensor in MEMORY order: dims string = layout (optionally with letters renamed), contiguous strides.
   sb_tensor mem(const void* ptr, const std::string& dims) const {
     sb_tensor t;
@@ -921,6 +926,7 @@ int einsum_fused(sb_encoder* e, cudaStream_t s, const char* name, Contract which
   if (ep->dropout) SB_TRY(to_rng(ep->dropout, &k.epi.rng));
   k.epi.skip_c = ep->discard_c ? 1 : 0;
   k.epi.skip_out2 = keep ? 0 : 1;
+  k.epi.few_tiles = e->private_pass ? 1 : 0;   // ordinary passes keep their operators separate at small sizes
   if (!keep && ep->dropout && ep->dropout->mode == SB_MASK_PHILOX) k.epi.mask = nullptr;
   e->mark(s, name);
   const int st = run_einsum_fused(s, k.g, k.epi);
@@ -1169,9 +1175,10 @@ static int forward_pass(sb_encoder* e, void* stream, const void* x, const void* 
   SB_TRY(gather(e, x, params, fwd, &T));
   T[TID("SB2")] = y;
   e->launches = 0;
+  e->private_pass = priv != nullptr;
   e->kernel_base = g_kernel_launches;
   auto L = [&](int id) -> const std::string& { return e->dims[id]; };
-  const long long slice = (long long)e->P * e->H * e->B * e->S;  // elements per stacked projection
+  const long long slice = e->slice();  // elements per stacked projection
   auto q_slice = [&](int q) { return (void*)((sb_half*)T[TID("KKQQVV")] + q * slice); };
   auto lKK = [&] { return L(TID("KKQQVV")).substr(1); };
 
@@ -1331,9 +1338,10 @@ static int backward_pass(sb_encoder* e, void* stream, const void* dy, void* cons
     D[e->param_order[i]] = dparams[i];
   }
   e->launches = 0;
+  e->private_pass = priv != nullptr;
   e->kernel_base = g_kernel_launches;
   auto L = [&](int id) -> const std::string& { return e->dims[id]; };
-  const long long slice = (long long)e->P * e->H * e->B * e->S;
+  const long long slice = e->slice();
   auto q_slice = [&](void* base, int q) { return (void*)((sb_half*)base + q * slice); };
   auto lKK = [&] { return L(TID("KKQQVV")).substr(1); };
   auto lDKK = [&] { return L(TID("DKKQQVV")).substr(1); };

@@ -685,6 +685,7 @@ splitk_reduce_kernel(const float* __restrict__ ws, int splits, long long batch, 
 
 #include "gemm_pair.cuh"
 #include "gemm_pair_splitk.cuh"
+#include "gemm_cluster_splitk.cuh"
 #include "attn_fused.cuh"
 #include "score_contract.cuh"
 #include "flash_attn.cuh"
@@ -1045,6 +1046,72 @@ int launch_tc_pair_splitk(cudaStream_t s, const GemmProblem& g, const OperandMap
   return SB_OK;
 }
 
+// Single-CTA split-K clusters for problems with a short side: how many CTAs share a tile's K (0: not this kernel).
+// Up to 256 rows or columns: beyond that the paired kernel and its split-K form have tiles enough (at 512 tokens they are
+// as fast).  Two CTAs fit on an SM, every CTA keeps two K blocks, and clusters of eight were slower than of four whenever
+// both fit (barriers and remote reads: 10.5 against 6.8 us for `out` at 256 tokens, 15.7 against 12.3 us for dXlin1).
+// Contractions and elementwise operators of an inference pass at 1024 features, together: 40.3 -> 35.4 us at 128 tokens,
+// 58.4 -> 37.0 at 200, 46.4 -> 37.6 at 256; of a training step 104.8 -> 95.5, 135 -> 106, 118.8 -> 105.6 us.
+int cluster_splits(const GemmProblem& g) {
+  if (g.batch != 1 || g.sCn != 1 || std::min(g.M, g.N) > 256 || g.sCm % 8 != 0 || (reinterpret_cast<uintptr_t>(g.C) & 15u))
+    return 0;
+  const long long tiles = ((g.M + kBM - 1) / kBM) * ((g.N + csk::kBN - 1) / csk::kBN), KT = (g.K + kBK - 1) / kBK;
+  const int sms = sm_count();
+  for (int sk : {4, 2})
+    if (tiles * sk <= 2 * sms && KT >= 2 * sk) return sk;
+  return 0;
+}
+
+// C^T = B^T A^T
+void transpose_problem(GemmProblem* g) {
+  std::swap(g->M, g->N);
+  std::swap(g->A, g->B);
+  std::swap(g->sAb, g->sBb);
+  std::swap(g->sAm, g->sBn);
+  std::swap(g->sAk, g->sBk);
+  std::swap(g->sCm, g->sCn);
+}
+
+template <int SK>
+int launch_cluster_splitk(cudaStream_t s, const GemmProblem& g, const OperandMap& a, const OperandMap& b, const GemmEpilogue* epi,
+                          bool vec_flipped) {
+  TcParams p;
+  memset(&p, 0, sizeof(p));
+  p.M = g.M; p.N = g.N; p.K = g.K;
+  p.sCm = g.sCm; p.sCn = 1;
+  p.C = g.C;
+  p.alpha = g.alpha;
+  p.a_mn = a.mn; p.b_mn = b.mn; p.a_swap = a.swap; p.b_swap = b.swap;
+  p.tiles_n = (int)((g.N + csk::kBN - 1) / csk::kBN);
+  p.tiles_m = (int)((g.M + kBM - 1) / kBM);
+  p.batch = 1;
+  p.kt_per_split = (int)(((g.K + kBK - 1) / kBK + SK - 1) / SK);
+  p.tiles = (long long)p.tiles_m * p.tiles_n;
+  csk::Outs o{reinterpret_cast<sb_half*>(g.C), nullptr, nullptr};
+  if (epi) {
+    auto misaligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) != 0; };
+    p.epi.kind = epi->kind;
+    p.epi.vec_along_m = vec_flipped ? !epi->vec_along_m : epi->vec_along_m;
+    if (epi->kind < 1 || epi->kind > 3 || (g.N % 8 != 0 && !(epi->kind == 1 && p.epi.vec_along_m)) || misaligned(epi->out2) || (epi->kind == 3 && misaligned(epi->out3)) ||
+        (epi->kind != 2 && !p.epi.vec_along_m && misaligned(epi->vec)) || (epi->kind == 2 && misaligned(epi->resid)) ||
+        (epi->kind == 3 && (reinterpret_cast<uintptr_t>(epi->mask) & 7u)))
+      return fail(SB_ERR_UNSUPPORTED, "fused epilogue: not one the split-K cluster kernel takes");
+    p.epi.vec = reinterpret_cast<const sb_half*>(epi->vec);
+    p.epi.resid = reinterpret_cast<const sb_half*>(epi->resid);
+    p.epi.mask = reinterpret_cast<uint8_t*>(epi->mask);
+    p.epi.activation = epi->activation;
+    p.epi.skip_c = epi->skip_c;
+    p.epi.skip_out2 = epi->skip_out2;
+    p.epi.rng = epi->rng;
+    o.out2 = reinterpret_cast<sb_half*>(epi->out2);
+    o.out3 = reinterpret_cast<sb_half*>(epi->out3);
+  }
+  const auto kernel = csk::gemm_cluster_splitk_kernel<SK>;
+  SB_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), csk::kSmemBytes));
+  SB_LAUNCH_OK(launch_k(kernel, (unsigned)(p.tiles * SK), csk::kThreads, csk::kSmemBytes, s, a.map, b.map, p, o));
+  return SB_OK;
+}
+
 int pick_bn(long long M, long long N, long long batch) {
   // 128 x 256 moves the fewest operand bytes per flop (each CTA fetches its own tiles), so it is
   // used whenever N fills most of it and the persistent grid still covers about half the SMs
@@ -1081,22 +1148,28 @@ int launch_gemm_tcgen05_epi(cudaStream_t s, const GemmProblem& g0, void* ws, siz
   if (!tcgen05_supported(g0, &why)) return fail(SB_ERR_UNSUPPORTED, "tcgen05 contraction: " + why);
   std::call_once(g_encode_once, load_encode);
   if (!g_encode) return fail(SB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+  OperandMap a, b;
+  {
+    GemmProblem gs = g0;                       // C's rows are the stored lines
+    const bool flip = g0.sCn != 1 && g0.sCm == 1;
+    if (flip) transpose_problem(&gs);
+    if (const int sk = epi && !epi->few_tiles ? 0 : cluster_splits(gs)) {
+      if (make_operand_map(gs.A, gs.M, gs.K, 1, gs.sAm, gs.sAk, gs.sAb, kBM, &a, &why) &&
+          make_operand_map(gs.B, gs.N, gs.K, 1, gs.sBn, gs.sBk, gs.sBb, csk::kBN, &b, &why)) {
+        const int st2 = sk == 4 ? launch_cluster_splitk<4>(s, gs, a, b, epi, flip) : launch_cluster_splitk<2>(s, gs, a, b, epi, flip);
+        if (st2 == SB_OK) g_last_gemm_impl = SB_GEMM_TCGEN05;
+        if (st2 != SB_ERR_UNSUPPORTED) return st2;
+      }
+    }
+  }
   // C^T = B^T A^T: use the orientation that wastes fewer padded tile elements
   // (ties: keep N as the unit-stride index of C so rows are stored as full lines).
   GemmProblem g = g0;
   const long long w0 = padded_work(g.M, g.N), w1 = padded_work(g.N, g.M);
   // With fused epilogue work the rows of C have to be the stored lines.
   const bool swap = epi ? g.sCn != 1 && g.sCm == 1 : (w1 < w0) || (w1 == w0 && g.sCn != 1 && g.sCm == 1);
-  if (swap) {
-    std::swap(g.M, g.N);
-    std::swap(g.A, g.B);
-    std::swap(g.sAb, g.sBb);
-    std::swap(g.sAm, g.sBn);
-    std::swap(g.sAk, g.sBk);
-    std::swap(g.sCm, g.sCn);
-  }
+  if (swap) transpose_problem(&g);
   const int bn = pick_bn(g.M, g.N, g.batch);
-  OperandMap a, b;
   // Large single-batch problems go to the paired-CTA kernel (256 x 256 tiles) when enough of its
   // clusters fit on the device and there are enough tiles to keep them busy.
   if (bn == 256 && g.batch == 1 && g.M >= 256 && g.N >= 256 && g.K >= 256 && pair_enabled()) {

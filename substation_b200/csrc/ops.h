@@ -116,6 +116,7 @@ struct GemmEpilogue {
   void* out2;
   void* out3;
   int skip_c;          // do not store C itself (only the fused outputs are wanted)
+  int few_tiles;       // the split-K cluster kernel may take it too (else only the paired-CTA kernel)
   float* partial;      // kind 4: [gemm_row_blocks(M)][N] column sums of out2 over blocks of 32 rows
   int skip_out2;       // kind 3: do not store out2, nor (mask null) a generated mask
 };
