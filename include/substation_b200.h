@@ -363,7 +363,8 @@ int sb_encoder_backward(sb_encoder* enc, void* stream, const void* dy, void* con
  * passes do not apply: fusion off, dead stores on, head size other than 64, or layouts the kernels do not read (the
  * passes themselves then return SB_ERR_UNSUPPORTED for the last two).  A backward pass takes the scratch of its forward
  * pass, which must have run with keep != 0, and that pass's mask mode; scratch is 16-byte aligned.  Intermediates are kept in
- * orders of the library's choosing (same sizes); x, y, dy, dx, parameters, their gradients and explicit masks keep the
+ * orders of the library's choosing (same sizes, except that KKQQVV, WKKWQQWVV, GAMMA, DGAMMA and DKKQQVV hold rows of B * S
+ * rounded up to a multiple of 8); x, y, dy, dx, parameters, their gradients and explicit masks keep the
  * configured ones. */
 int sb_encoder_private_bytes(sb_encoder* enc, int mask_mode, size_t* forward, size_t* backward);
 int sb_encoder_forward_private(sb_encoder* enc, void* stream, const void* x, const void* const* params,

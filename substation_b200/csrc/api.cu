@@ -774,7 +774,9 @@ struct sb_encoder {
     t.ptr = const_cast<void*>(ptr);
     t.ndim = (int)dims.size();
     long long st = 1;
+    const bool padded = token_pitch && t.ndim > 3 && dims.compare(t.ndim - 3, 2, "HB") == 0;
     for (int i = t.ndim - 1; i >= 0; --i) {
+      if (padded && i == t.ndim - 3) st = token_pitch;
       t.size[i] = extent(dims[i]);
       t.stride[i] = st;
       st *= t.size[i];
@@ -1023,7 +1025,9 @@ extern "C" int sb_encoder_create(const sb_encoder_config* cfg, sb_encoder** out)
     SB_CUDA_OK(cudaMalloc(&e->workspace, kWsBytes));
   }
   SB_CUDA_OK(cudaMemset(e->workspace, 0, kWsCounterBytes));   // the partial sums behind the counters need no value
-  if (!features_innermost(e.get())) {
+  // (score tensors have no part in private passes, so the pitch of ..HBJ never meets HBJK)
+  const bool ragged = (long long)e->B * e->S % 8 != 0;
+  if (!features_innermost(e.get()) || ragged) {
     e->twin.reset(new sb_encoder);
     sb_encoder* t = e->twin.get();
     t->B = e->B; t->S = e->S; t->H = e->H; t->I = e->I; t->P = e->P; t->U = e->U;
@@ -1034,6 +1038,7 @@ extern "C" int sb_encoder_create(const sb_encoder_config* cfg, sb_encoder** out)
     for (const char* n : kParamNames) t->layout[n] = e->layout.at(n);
     t->workspace = e->workspace; t->gemm_ws = e->gemm_ws; t->gemm_ws_bytes = e->gemm_ws_bytes;   // owned by e
     t->device = e->device;
+    if (ragged) t->token_pitch = ((long long)e->B * e->S + 7) / 8 * 8;
     derive(t);
   }
   *out = e.release();
@@ -1688,8 +1693,7 @@ sb_encoder* private_target(sb_encoder* e, int mask_mode) {
 
 int private_supported(const sb_encoder* e, const sb_encoder* t) {
   if (e->dims[TID("ATTN_DROP_MASK")] != "HBJK" ||
-      flash_supported(e->H, e->B, e->S, e->P, proj_view(t->proj), proj_view(t->dproj), proj_view(t->logical[TID("GAMMA")]),
-                      proj_view(t->logical[TID("DGAMMA")])) != SB_OK)
+      flash_supported(e->H, e->B, e->S, e->P, proj_view(t->proj), proj_view(t->logical[TID("DGAMMA")])) != SB_OK)
     return fail(SB_ERR_UNSUPPORTED, "private passes need head size 64, score masks stored as HBJK and projections with unit "
                                     "stride along the head or the sequence dim");
   return SB_OK;
@@ -1699,7 +1703,8 @@ int private_supported(const sb_encoder* e, const sb_encoder* t) {
 struct PrivateScratch { size_t attn_fwd, attn_bwd, act; };
 PrivateScratch private_scratch(const sb_encoder* e, const sb_encoder* t) {
   FlashScratch f;
-  flash_scratch(e->H, e->B, e->S, flash_padded(proj_view(t->proj), e->S), flash_padded(proj_view(t->logical[TID("DGAMMA")]), e->S), &f);
+  flash_scratch(e->H, e->B, e->S, flash_padded(proj_view(t->proj), e->H, e->B, e->S),
+                flash_padded(proj_view(t->logical[TID("DGAMMA")]), e->H, e->B, e->S), &f);
   const size_t act = t->dims[TID("X")] != e->dims[TID("X")] ? ((size_t)e->B * e->S * e->I * sizeof(sb_half) + 255) / 256 * 256 : 0;
   return PrivateScratch{f.fwd_bytes, f.bwd_bytes, act};
 }

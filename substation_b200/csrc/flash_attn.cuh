@@ -183,7 +183,8 @@ struct FwdParams {
   uint4* bits;             // [unit][nb][L] words of 128 flags, or null
   float* lse;              // [unit][L], or null
   sb_half* out;
-  long long o_sU, o_sRow, o_sP;
+  int B;                   // unit u is head u / B of sample u % B
+  long long o_sH, o_sB, o_sRow, o_sP;
 };
 
 // One CTA: 128 query rows of one unit against all keys in tiles of 128; two CTAs per SM, so that one's tensor and
@@ -434,7 +435,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       __syncwarp();
       if (lane == 0) mbar_arrive(o_empty);
       if (row) {
-        store_cols<64>(p.out + (long long)u * p.o_sU + (long long)j * p.o_sRow, p.o_sP, r, 1.f / l);
+        store_cols<64>(p.out + (u / p.B) * p.o_sH + (u % p.B) * p.o_sB + (long long)j * p.o_sRow, p.o_sP, r, 1.f / l);
         if (p.lse) p.lse[(long long)u * L + j] = (m == -INFINITY ? 0.f : m * p.c2) + log2f(l);
       }
     }
@@ -464,7 +465,8 @@ struct BwdParams {
   const float* lse;
   const float* dsum;       // [unit][L]: sum_p DGAMMA * GAMMA = sum_k ALPHA * dALPHA
   sb_half* dq; sb_half* dk; sb_half* dv;
-  long long d_sU, d_sRow, d_sP;
+  int B;
+  long long d_sH, d_sB, d_sRow, d_sP;
 };
 
 // Which of the four tile-pair slots are used for what: one is held for a whole item, the other three take the tiles
@@ -652,7 +654,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       const uint32_t acc = tmem_acc + set * 128u + lanes;
       const bool qi = is_q(item);
       const int u = unit_of(item), r0 = block_of(item) * 128 + rt;
-      const long long off = (long long)u * p.d_sU + (long long)r0 * p.d_sRow;
+      const long long off = (u / p.B) * p.d_sH + (u % p.B) * p.d_sB + (long long)r0 * p.d_sRow;
       // 32 columns at a time: two pieces of dV (h = 0) or dK (h = 1), one of dQ
 #pragma unroll 1
       for (int c = qi ? 2 : 0; c < (qi || p.both ? 3 : 2); ++c) {
@@ -768,15 +770,16 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 }
 
 // ---- small kernels around them ---------------------------------------------------------------------------------
-// Row-contiguous projections whose rows do not start on 16-byte boundaries (L not a multiple of 8) are copied to
-// [p][unit][Lp] with Lp = L rounded up to 8, which tensor maps can address.
+// Row-contiguous projections whose rows do not start on 16-byte boundaries (L not a multiple of 8), or whose head and
+// sample dims do not collapse, are copied to [p][unit][Lp] with Lp = L rounded up to 8, which tensor maps can address.
 __global__ void __launch_bounds__(256)
-pad_projections_kernel(const sb_half* src, long long slice, long long sP, long long sU, sb_half* dst, int units, int L, int Lp) {
+pad_projections_kernel(const sb_half* src, long long slice, long long sP, long long sH, long long sB, int B, sb_half* dst, int units,
+                       int L, int Lp) {
   grid_dependency_sync();
   const long long rows = 192ll * units;
   for (long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += (long long)gridDim.x * 8) {
     const int pp = (int)(r / units), u = (int)(r % units);
-    const sb_half* s = src + (pp >> 6) * slice + (pp & 63) * sP + u * sU;
+    const sb_half* s = src + (pp >> 6) * slice + (pp & 63) * sP + (u / B) * sH + (u % B) * sB;
     sb_half* d = dst + r * Lp;
     for (int j = threadIdx.x & 31; j < L; j += 32) d[j] = s[j];
   }
@@ -785,11 +788,11 @@ pad_projections_kernel(const sb_half* src, long long slice, long long sP, long l
 // dsum[unit][j] = sum_p DGAMMA * GAMMA, 32 rows per block, eight head-dim indices per thread; with `pad`, DGAMMA is
 // copied as above on the way.
 struct DsumParams {
-  const sb_half* g; long long g_sP, g_sU, g_sRow;
-  const sb_half* o; long long o_sP, o_sU, o_sRow;
+  const sb_half* g; long long g_sP, g_sH, g_sB, g_sRow;
+  const sb_half* o; long long o_sP, o_sH, o_sB, o_sRow;
   float* dsum;
   sb_half* pad;
-  int units, L, Lp, blocks_j;
+  int units, B, L, Lp, blocks_j;
 };
 __global__ void __launch_bounds__(256)
 dsum_kernel(const DsumParams p) {
@@ -797,13 +800,14 @@ dsum_kernel(const DsumParams p) {
   grid_dependency_sync();
   const int u = (int)(blockIdx.x / p.blocks_j), j = (int)(blockIdx.x % p.blocks_j) * 32 + (threadIdx.x & 31);
   const int pg = threadIdx.x >> 5;
+  const long long g0 = (u / p.B) * p.g_sH + (u % p.B) * p.g_sB + j * p.g_sRow, o0 = (u / p.B) * p.o_sH + (u % p.B) * p.o_sB + j * p.o_sRow;
   float acc = 0.f;
   if (j < p.L) {
     sb_half g[8], o[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      g[e] = p.g[(pg * 8 + e) * p.g_sP + u * p.g_sU + j * p.g_sRow];
-      o[e] = p.o[(pg * 8 + e) * p.o_sP + u * p.o_sU + j * p.o_sRow];
+      g[e] = p.g[(pg * 8 + e) * p.g_sP + g0];
+      o[e] = p.o[(pg * 8 + e) * p.o_sP + o0];
     }
 #pragma unroll
     for (int e = 0; e < 8; ++e) {

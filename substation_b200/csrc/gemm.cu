@@ -815,14 +815,14 @@ int launch_tc(cudaStream_t s, const GemmProblem& g, const OperandMap& a, const O
   p.tiles = base_tiles * p.splits;
   CUtensorMap cmap;
   memset(&cmap, 0, sizeof(cmap));
-  const bool c_vec = g.sCn == 1 && g.N % 8 == 0 && g.sCm % 8 == 0 && (g.batch == 1 || g.sCb % 8 == 0) &&
-                     (reinterpret_cast<uintptr_t>(g.C) & 15u) == 0;
+  // tensor-map stores clip at N; the plain 128-bit ones need it to be a multiple of 8
+  const bool c_tma = g.sCn == 1 && g.sCm % 8 == 0 && (g.batch == 1 || g.sCb % 8 == 0) && (reinterpret_cast<uintptr_t>(g.C) & 15u) == 0;
   if (p.splits > 1) {
     p.c_mode = 3;
     p.C = ws;
   } else {
-    p.c_mode = c_vec ? 1 : 0;
-    if (c_vec) {
+    p.c_mode = c_tma && g.N % 8 == 0 ? 1 : 0;
+    if (c_tma) {
       std::string why;
       int swapped = 0;
       if (encode_map(g.C, (cuuint64_t)g.N, (cuuint64_t)g.M, (cuuint64_t)g.batch, g.sCm, g.sCb, 64, 32, &cmap, &swapped, &why)) {
@@ -911,10 +911,9 @@ int launch_tc_pair(cudaStream_t s, const GemmProblem& g, const OperandMap& a, co
   p.tiles = (long long)p.tiles_m * p.tiles_n * g.batch;
   CUtensorMap cmap;
   memset(&cmap, 0, sizeof(cmap));
-  const bool c_vec = g.sCn == 1 && g.N % 8 == 0 && g.sCm % 8 == 0 && (g.batch == 1 || g.sCb % 8 == 0) &&
-                     (reinterpret_cast<uintptr_t>(g.C) & 15u) == 0;
-  p.c_mode = c_vec ? 1 : 0;
-  if (c_vec) {
+  const bool c_tma = g.sCn == 1 && g.sCm % 8 == 0 && (g.batch == 1 || g.sCb % 8 == 0) && (reinterpret_cast<uintptr_t>(g.C) & 15u) == 0;
+  p.c_mode = c_tma && g.N % 8 == 0 ? 1 : 0;
+  if (c_tma) {
     std::string why;
     int swapped = 0;
     if (encode_map(g.C, (cuuint64_t)g.N, (cuuint64_t)g.M, (cuuint64_t)g.batch, g.sCm, g.sCb, 64, 32, &cmap, &swapped, &why)) {
@@ -928,8 +927,9 @@ int launch_tc_pair(cudaStream_t s, const GemmProblem& g, const OperandMap& a, co
   memset(&cmap2, 0, sizeof(cmap2));
   memset(&cmap3, 0, sizeof(cmap3));
   if (epi) {
-    // fused epilogue work needs the TMA-store path and whole 64-column blocks
-    if (p.c_mode != 2 || g.N % 64 != 0)
+    // fused epilogue work needs the TMA-store path, and whole 64-column blocks where it reads anything along them
+    const bool along_m = vec_flipped ? !epi->vec_along_m : epi->vec_along_m;
+    if (p.c_mode != 2 || (g.N % 64 != 0 && !(epi->kind == 1 && along_m)))
       return fail(SB_ERR_UNSUPPORTED, "fused epilogue: output rows must be TMA-addressable with N a multiple of 64");
     std::string why;
     int sw = 0;
@@ -1393,12 +1393,14 @@ int launch_score_contract(cudaStream_t s, Dims4 d, int P, View4 scores, const Vi
 
 namespace {
 
-// [P,H,B,rows] projection (View4 fields hold the P,H,B,row strides) as rows of units h * B + b.
-struct UnitView { long long sP, sU, sRow; };
-bool unit_view(const View4& v, int H, int B, UnitView* o) {
-  if (H > 1 && B > 1 && v.sB != v.sJ * B) return false;
-  o->sP = v.sH; o->sU = B > 1 ? v.sJ : v.sB; o->sRow = v.sK;
-  return true;
+// [P,H,B,rows] projection (View4 fields hold the P,H,B,row strides): rows of units h * B + b, sU apart if they collapse.
+struct UnitView { long long sP, sH, sB, sU, sRow; bool collapses; };
+UnitView unit_view(const View4& v, int H, int B) {
+  UnitView o;
+  o.sP = v.sH; o.sH = v.sB; o.sB = v.sJ; o.sRow = v.sK;
+  o.collapses = H == 1 || B == 1 || v.sB == v.sJ * B;
+  o.sU = B > 1 ? v.sJ : v.sB;
+  return o;
 }
 // Tensor map of a projection the flash kernels read in 64 x 64 boxes: `jc` when the rows are the unit-stride index.
 bool flash_map(const void* ptr, const UnitView& v, int units, int L, CUtensorMap* map, int* jc, int* swap, std::string* why) {
@@ -1409,19 +1411,23 @@ bool flash_map(const void* ptr, const UnitView& v, int units, int L, CUtensorMap
 }
 long long pad8(long long n) { return (n + 7) / 8 * 8; }
 size_t align256(size_t n) { return (n + 255) / 256 * 256; }
+// what a padded copy looks like
+void padded_view(UnitView* v, int units, int L) {
+  v->sRow = 1; v->sU = pad8(L); v->sP = v->sU * units;
+}
 
 }  // namespace
 
-// Rows of the projections are the unit-stride index and not 16 bytes apart: the kernels read a padded copy.
-bool flash_padded(const View4& v, int L) { return v.sK == 1 && v.sH != 1 && L % 8 != 0; }
+// The rows are the projections' unit-stride index and units are not 16 bytes apart, or not in one sequence: the kernels
+// read a padded copy.
+bool flash_padded(const View4& v, int H, int B, int L) {
+  return v.sK == 1 && v.sH != 1 && (L % 8 != 0 || !unit_view(v, H, B).collapses);
+}
 
-int flash_supported(int H, int B, int L, int P, View4 proj, View4 dproj, View4 gamma, View4 dgamma) {
-  UnitView u;
-  for (const View4* v : {&proj, &dproj, &gamma, &dgamma})
-    if (!unit_view(*v, H, B, &u)) return SB_ERR_UNSUPPORTED;
+int flash_supported(int H, int B, int L, int P, View4 proj, View4 dgamma) {
   for (const View4* v : {&proj, &dgamma}) {
     if (v->sH != 1 && v->sK != 1) return SB_ERR_UNSUPPORTED;
-    if (v->sH == 1 && ((v->sK | v->sJ | v->sB) & 7)) return SB_ERR_UNSUPPORTED;
+    if (v->sH == 1 && (((v->sK | v->sJ | v->sB) & 7) || !unit_view(*v, H, B).collapses)) return SB_ERR_UNSUPPORTED;
   }
   if (P != 64 || L < 1 || (long long)H * B * ((L + 31) / 32) > 0x3fffffffLL) return SB_ERR_UNSUPPORTED;
   return SB_OK;
@@ -1442,18 +1448,18 @@ int launch_flash_fwd(cudaStream_t s, int H, int B, int L, const void* kqv, long 
   if (!g_encode) return fail(SB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   const int units = H * B;
   FlashScratch f;
-  const bool pad = flash_padded(proj, L);
+  const bool pad = flash_padded(proj, H, B, L);
   flash_scratch(H, B, L, pad, false, &f);
   char* sc = reinterpret_cast<char*>(scratch);
-  UnitView v, o;
-  if (!unit_view(proj, H, B, &v) || !unit_view(gv, H, B, &o)) return fail(SB_ERR_UNSUPPORTED, "attention: head and sample dims do not collapse");
+  UnitView v = unit_view(proj, H, B);
+  const UnitView o = unit_view(gv, H, B);
   const sb_half* base = reinterpret_cast<const sb_half*>(kqv);
   if (pad) {
     sb_half* dst = reinterpret_cast<sb_half*>(sc + f.pad);
     const unsigned grid = (unsigned)std::min<long long>((192ll * units + 7) / 8, (long long)sm_count() * 8);
-    SB_LAUNCH_OK(launch_k(flash::pad_projections_kernel, grid, 256, 0, s, base, slice, v.sP, v.sU, dst, units, L, (int)pad8(L)));
+    SB_LAUNCH_OK(launch_k(flash::pad_projections_kernel, grid, 256, 0, s, base, slice, v.sP, v.sH, v.sB, B, dst, units, L, (int)pad8(L)));
     base = dst;
-    v.sRow = 1; v.sU = pad8(L); v.sP = v.sU * units;
+    padded_view(&v, units, L);
     slice = 64 * v.sP;
   }
   flash::FwdParams p;
@@ -1469,7 +1475,8 @@ int launch_flash_fwd(cudaStream_t s, int H, int B, int L, const void* kqv, long 
   p.mask = reinterpret_cast<const uint8_t*>(mask);
   if (keep) { p.lse = reinterpret_cast<float*>(sc); p.bits = reinterpret_cast<uint4*>(sc + f.bits); }
   p.out = reinterpret_cast<sb_half*>(gamma);
-  p.o_sU = o.sU; p.o_sRow = o.sRow; p.o_sP = o.sP;
+  p.B = B;
+  p.o_sH = o.sH; p.o_sB = o.sB; p.o_sRow = o.sRow; p.o_sP = o.sP;
   const bool none = rng.philox && rng.thr == 0;
   auto kernel = none ? flash::flash_fwd_kernel<flash::kNoDrop>
                      : rng.philox && L % 8 == 0 ? flash::flash_fwd_kernel<flash::kPhilox> : flash::flash_fwd_kernel<flash::kAnyMask>;
@@ -1486,31 +1493,30 @@ int launch_flash_bwd(cudaStream_t s, int H, int B, int L, const void* kqv, long 
   if (!g_encode) return fail(SB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   const int units = H * B;
   FlashScratch f;
-  const bool pad = flash_padded(proj, L), dpad = flash_padded(dgv, L);
+  const bool pad = flash_padded(proj, H, B, L), dpad = flash_padded(dgv, H, B, L);
   flash_scratch(H, B, L, pad, dpad, &f);
   const char* fs = reinterpret_cast<const char*>(fwd_scratch);
   char* bs = reinterpret_cast<char*>(bwd_scratch);
-  UnitView v, o, g, d;
-  if (!unit_view(proj, H, B, &v) || !unit_view(gv, H, B, &o) || !unit_view(dgv, H, B, &g) || !unit_view(dproj, H, B, &d))
-    return fail(SB_ERR_UNSUPPORTED, "attention: head and sample dims do not collapse");
+  UnitView v = unit_view(proj, H, B), g = unit_view(dgv, H, B);
+  const UnitView o = unit_view(gv, H, B), d = unit_view(dproj, H, B);
   const sb_half* base = reinterpret_cast<const sb_half*>(kqv);
   if (pad) {
     base = reinterpret_cast<const sb_half*>(fs + f.pad);
-    v.sRow = 1; v.sU = pad8(L); v.sP = v.sU * units;
+    padded_view(&v, units, L);
     slice = 64 * v.sP;
   }
   flash::DsumParams q;
   memset(&q, 0, sizeof(q));
-  q.g = reinterpret_cast<const sb_half*>(dgamma); q.g_sP = g.sP; q.g_sU = g.sU; q.g_sRow = g.sRow;
-  q.o = reinterpret_cast<const sb_half*>(gamma); q.o_sP = o.sP; q.o_sU = o.sU; q.o_sRow = o.sRow;
+  q.g = reinterpret_cast<const sb_half*>(dgamma); q.g_sP = g.sP; q.g_sH = g.sH; q.g_sB = g.sB; q.g_sRow = g.sRow;
+  q.o = reinterpret_cast<const sb_half*>(gamma); q.o_sP = o.sP; q.o_sH = o.sH; q.o_sB = o.sB; q.o_sRow = o.sRow;
   q.dsum = reinterpret_cast<float*>(bs);
   q.pad = dpad ? reinterpret_cast<sb_half*>(bs + f.dpad) : nullptr;
-  q.units = units; q.L = L; q.Lp = (int)pad8(L); q.blocks_j = (L + 31) / 32;
+  q.units = units; q.B = B; q.L = L; q.Lp = (int)pad8(L); q.blocks_j = (L + 31) / 32;
   SB_LAUNCH_OK(launch_k(flash::dsum_kernel, (unsigned)((long long)units * q.blocks_j), 256, 0, s, q));
   const void* gptr = dgamma;
   if (dpad) {
     gptr = q.pad;
-    g.sRow = 1; g.sU = q.Lp; g.sP = g.sU * units;
+    padded_view(&g, units, L);
   }
   flash::BwdParams p;
   memset(&p, 0, sizeof(p));
@@ -1530,7 +1536,8 @@ int launch_flash_bwd(cudaStream_t s, int H, int B, int L, const void* kqv, long 
   p.dsum = q.dsum;
   sb_half* dk = reinterpret_cast<sb_half*>(dkqv);
   p.dk = dk; p.dq = dk + dslice; p.dv = dk + 2 * dslice;
-  p.d_sU = d.sU; p.d_sRow = d.sRow; p.d_sP = d.sP;
+  p.B = B;
+  p.d_sH = d.sH; p.d_sB = d.sB; p.d_sRow = d.sRow; p.d_sP = d.sP;
   static_assert(flash::kBwdSmem <= 232448, "shared memory of the attention backward kernel");
   SB_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(flash::flash_bwd_kernel), flash::kBwdSmem));
   const unsigned grid = (unsigned)std::min<long long>(p.items, sm_count());

@@ -82,8 +82,8 @@ struct FlashScratch {
   size_t bits, pad, fwd_bytes;   // forward: log-sum-exps at 0, then mask bits, then padded projections
   size_t dpad, bwd_bytes;        // backward: row sums at 0, then padded DGAMMA
 };
-int flash_supported(int H, int B, int L, int P, View4 proj, View4 dproj, View4 gamma, View4 dgamma);
-bool flash_padded(const View4& v, int L);
+int flash_supported(int H, int B, int L, int P, View4 proj, View4 dgamma);
+bool flash_padded(const View4& v, int H, int B, int L);
 void flash_scratch(int H, int B, int L, bool pad_proj, bool pad_dgamma, FlashScratch* f);
 int launch_flash_fwd(cudaStream_t s, int H, int B, int L, const void* kqv, long long slice, View4 proj, void* gamma, View4 gv,
                      const void* mask, float scale, Rng rng, void* scratch, bool keep);

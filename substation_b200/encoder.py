@@ -388,6 +388,9 @@ class Encoder(torch.nn.Module):
     # attention intermediates a private pass does without
     _SCORES = frozenset(('BETA', 'ALPHA', 'ATTN_DROP', 'ATTN_DROP_MASK', 'DATTN_DROP', 'DBETA'))
 
+    # tensors whose rows are all tokens: a private pass pads them to a multiple of 8
+    _HEAD_FIRST = frozenset(('KKQQVV', 'WKKWQQWVV', 'GAMMA', 'DGAMMA', 'DKKQQVV'))
+
     def _private_plans(self, device):
         """Arena plans of a pass whose intermediates nobody looks at (score tensors without storage, the library's
         scratch behind the others), or None where the library has no such pass for this configuration."""
@@ -403,11 +406,12 @@ class Encoder(torch.nn.Module):
         cached = self.__dict__.get('_private')
         if cached is None or cached['key'] != key:
             cached = {'key': key, 'mask_mode': mode}
+            tokens = self.batch_size * self.max_seq_len
             for which, entries, extra in (('fwd', self.layouts['forward_interm'], nf.value),
                                           ('bwd', self.layouts['backward_interm'], nb.value)):
                 plan, off = [], 0
                 for name, shape, dtype, _, nbytes in self._plan(entries)[0]:
-                    n = 0 if name in self._SCORES else nbytes
+                    n = 0 if name in self._SCORES else nbytes // tokens * _round_up(tokens, 8) if name in self._HEAD_FIRST else nbytes
                     plan.append((name, shape, dtype, off if n else 0, n))
                     off += _round_up(n)
                 cached[which], cached[which + '_scratch'] = (plan, off + extra), off

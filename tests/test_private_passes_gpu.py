@@ -32,8 +32,10 @@ def _passes(B, S, H, dtype, p, mode, lay, seed, activation='gelu'):
                       keep_all_intermediates=keep).to(dev)
         with torch.no_grad():
             if state is None:
+                # unit-variance projections: the keeping pass rounds the scores to 16 bits, an error in ALPHA of half a unit
+                # times the score, which the bound above counts once only because scores stay of order one
                 for q in enc.params:
-                    q.copy_((torch.randn(q.shape, device=dev, generator=gen) * 0.1).to(dtype))
+                    q.copy_((torch.randn(q.shape, device=dev, generator=gen) * (1.1 / E ** 0.5)).to(dtype))
                 enc.S1.fill_(1)
                 enc.S2.fill_(1)
                 state = enc.state_dict()
@@ -117,3 +119,37 @@ def test_row_maxima_that_rise_by_more_than_the_lag():
         assert torch.isfinite(b).all()
         # the keeping pass rounds scores of up to ~100 to 16 bits before exponentiating: errors of 2^-5 in ALPHA
         assert ((a.double() - b.double()).norm() / a.double().norm()).item() <= 2.0 ** -5
+
+
+@pytest.mark.parametrize('B,S,H,dtype,mode', [
+    (1, 19, 2, torch.float16, 'philox'),                             # all token counts off the 8 grid: rows of the
+    (1, 77, 8, torch.float16, 'explicit'),                           # head-first tensors are padded to it
+    (1, 130, 8, torch.bfloat16, 'philox'),
+    (5, 100, 16, torch.float16, 'philox'),
+    (3, 333, 8, torch.float16, 'philox'),
+])
+def test_token_counts_off_the_vector_grid(B, S, H, dtype, mode):
+    for layouts in ('uniform', 'feature_major'):
+        kept, private = _passes(B, S, H, dtype, 0.1, mode, cases._layouts({'layouts': layouts}), seed=S)
+        for name, want in kept.items():
+            err = ((private[name].double() - want.double()).norm() / want.double().norm()).item()
+            assert torch.isfinite(private[name]).all() and err <= 8 * HALF[dtype], (layouts, name, err)
+
+
+@pytest.mark.parametrize('M,N,K', [(128, 64, 256), (1, 1024, 512), (77, 1024, 1000), (256, 3072, 1024), (130, 520, 320),
+                                   (200, 72, 4096), (1024, 77, 1024)])
+def test_split_k_clusters(M, N, K):
+    """Contractions with a side of at most 256 against float64: edges of the 128 x 64 tile, K that does not divide among
+    the CTAs, both majors of both operands.  Bound: half a unit of the 16-bit result plus fp32 sums of K products."""
+    from substation_b200 import ops
+    dev = torch.device('cuda:0')
+    gen = torch.Generator(device=dev).manual_seed(M + N + K)
+    for am in (False, True):
+        for bm in (False, True):
+            a = torch.randn((K, M) if am else (M, K), device=dev, generator=gen).half()
+            b = torch.randn((K, N) if bm else (N, K), device=dev, generator=gen).half()
+            c = torch.zeros(M, N, device=dev, dtype=torch.float16)
+            ops.einsum(('km' if am else 'mk') + ',' + ('kn' if bm else 'nk') + '->mn', a, b, c)
+            want = (a.T if am else a).double() @ (b if bm else b.T).double()
+            err = ((c.double() - want).norm() / want.norm()).item()
+            assert err <= 2.0 ** -11 + K ** 0.5 * 2.0 ** -23, (am, bm, err)
