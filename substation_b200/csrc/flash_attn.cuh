@@ -825,4 +825,42 @@ dsum_kernel(const DsumParams p) {
   }
 }
 
+// The same where rows are consecutive and 16-byte aligned in both (L a multiple of 8): eight rows per access, 128 rows per
+// block, four head-dim indices per thread.  Two bytes at a time took 13.9 us for the 50 MB of B=96, L=128.
+__global__ void __launch_bounds__(256)
+dsum_vec_kernel(const DsumParams p) {
+  __shared__ float part[16][128 + 4];
+  grid_dependency_sync();
+  const int u = (int)(blockIdx.x / p.blocks_j), oct = threadIdx.x & 15, j = (int)(blockIdx.x % p.blocks_j) * 128 + oct * 8;
+  const int pg = threadIdx.x >> 4;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (j < p.L) {
+    const long long g0 = (u / p.B) * p.g_sH + (u % p.B) * p.g_sB + j, o0 = (u / p.B) * p.o_sH + (u % p.B) * p.o_sB + j;
+    uint4 g[4], o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      g[e] = *reinterpret_cast<const uint4*>(p.g + (pg * 4 + e) * p.g_sP + g0);
+      o[e] = *reinterpret_cast<const uint4*>(p.o + (pg * 4 + e) * p.o_sP + o0);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float a[8], b[8];
+      unpack8(g[e], a);
+      unpack8(o[e], b);
+#pragma unroll
+      for (int x = 0; x < 8; ++x) acc[x] = fmaf(a[x], b[x], acc[x]);
+    }
+  }
+#pragma unroll
+  for (int x = 0; x < 8; x += 4) *reinterpret_cast<float4*>(&part[pg][oct * 8 + x]) = make_float4(acc[x], acc[x + 1], acc[x + 2], acc[x + 3]);
+  __syncthreads();
+  const int r = (int)(blockIdx.x % p.blocks_j) * 128 + threadIdx.x;
+  if (threadIdx.x < 128 && r < p.L) {
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) s += part[i][threadIdx.x];
+    p.dsum[(long long)u * p.L + r] = s;
+  }
+}
+
 }  // namespace flash

@@ -1511,8 +1511,13 @@ int launch_flash_bwd(cudaStream_t s, int H, int B, int L, const void* kqv, long 
   q.o = reinterpret_cast<const sb_half*>(gamma); q.o_sP = o.sP; q.o_sH = o.sH; q.o_sB = o.sB; q.o_sRow = o.sRow;
   q.dsum = reinterpret_cast<float*>(bs);
   q.pad = dpad ? reinterpret_cast<sb_half*>(bs + f.dpad) : nullptr;
-  q.units = units; q.B = B; q.L = L; q.Lp = (int)pad8(L); q.blocks_j = (L + 31) / 32;
-  SB_LAUNCH_OK(launch_k(flash::dsum_kernel, (unsigned)((long long)units * q.blocks_j), 256, 0, s, q));
+  q.units = units; q.B = B; q.L = L; q.Lp = (int)pad8(L);
+  auto rows_of_eight = [&](const void* ptr, const UnitView& w) {
+    return w.sRow == 1 && !((w.sP | w.sH | w.sB) & 7) && !(reinterpret_cast<uintptr_t>(ptr) & 15u);
+  };
+  const bool vec = L % 8 == 0 && !dpad && rows_of_eight(dgamma, g) && rows_of_eight(gamma, o);
+  q.blocks_j = vec ? (L + 127) / 128 : (L + 31) / 32;
+  SB_LAUNCH_OK(launch_k(vec ? flash::dsum_vec_kernel : flash::dsum_kernel, (unsigned)((long long)units * q.blocks_j), 256, 0, s, q));
   const void* gptr = dgamma;
   if (dpad) {
     gptr = q.pad;
