@@ -125,7 +125,7 @@ class _EncoderFunction(torch.autograd.Function):
         g16 = garena[:max(gtotal, 2)].view(outer.torch_dtype)
         outer._grad_bucket = g16
         grads = tuple(torch.as_strided(g16, shape, strides, off) for shape, strides, off in outer._grad_views)
-        if outer.enable_debug:
+        if outer.enable_debug and not private:
             torch.cuda.synchronize()
             bwd = outer.views('backward', barena)
             for name in outer._bwd_names:
