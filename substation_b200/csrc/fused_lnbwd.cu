@@ -415,16 +415,21 @@ lnbwd_ring_kernel(LnBwdParams p, int nstages, int stage_bytes) {
   }
 }
 
-// out[q][f] = sum over the P partial rows in a fixed order: 16 thread groups take every 16th row each (loads
-// issued eight at a time, then added in row order) and are combined through shared memory in group order.
-constexpr int kFinishParts = 16;
-__global__ void __launch_bounds__(64 * kFinishParts)
-colsum_finish_kernel(const float* __restrict__ partial, int P, int F, int ld, void* o0, void* o1, void* o2, void* o3) {
+// out[q][f] = sum over the P partial rows in a fixed order: 32 warps take every 32nd row each (loads issued eight at a
+// time, then added in row order; a warp reads 32 features) and are combined through shared memory in warp order.  Bound by
+// the latency of its loads: the 148 rows of a full machine are one round of them (16 thread groups made it two).
+constexpr int kFinishParts = 32;
+constexpr int kFinishCols = 32;
+// LD: floats between partial rows, 0: F.
+template <int LD>
+__global__ void __launch_bounds__(kFinishCols * kFinishParts)
+colsum_finish_kernel(const float* __restrict__ partial, int P, int F, void* o0, void* o1, void* o2, void* o3) {
   grid_dependency_sync();
-  __shared__ float sm[kFinishParts][64];
+  __shared__ float sm[kFinishParts][kFinishCols];
+  const int ld = LD ? LD : F;
   const int q = blockIdx.y;
-  const int fl = threadIdx.x & 63, part = threadIdx.x >> 6;
-  const int f = blockIdx.x * 64 + fl;
+  const int fl = threadIdx.x % kFinishCols, part = threadIdx.x / kFinishCols;
+  const int f = blockIdx.x * kFinishCols + fl;
   float v = 0.f;
   if (f < F) {
     const float* base = partial + (long long)q * P * ld + f;
@@ -654,8 +659,8 @@ int launch(cudaStream_t s, void* ws, const LnBwdParams& p0, void* const outs[4])
     SB_LAUNCH_OK(launch_k(lnbwd_kernel<MODE>, P, kThreads, smem, s, p));
   }
   SB_CUDA_OK(cudaGetLastError());
-  dim3 grid((p.d.F + 63) / 64, NQ);
-  SB_LAUNCH_OK(launch_k(colsum_finish_kernel, grid, 64 * kFinishParts, 0, s, p.partial, P, p.d.F, kMaxF, outs[0], outs[1], outs[2], outs[3]));
+  dim3 grid((p.d.F + kFinishCols - 1) / kFinishCols, NQ);
+  SB_LAUNCH_OK(launch_k(colsum_finish_kernel<kMaxF>, grid, kFinishCols * kFinishParts, 0, s, p.partial, P, p.d.F, outs[0], outs[1], outs[2], outs[3]));
   SB_CUDA_OK(cudaGetLastError());
   return SB_OK;
 }
@@ -663,7 +668,7 @@ int launch(cudaStream_t s, void* ws, const LnBwdParams& p0, void* const outs[4])
 }  // namespace
 
 int launch_colsum(cudaStream_t s, const float* partial, int P, int F, void* out) {
-  SB_LAUNCH_OK(launch_k(colsum_finish_kernel, dim3((F + 63) / 64, 1), 64 * kFinishParts, 0, s, partial, P, F, F, out, nullptr, nullptr, nullptr));
+  SB_LAUNCH_OK(launch_k(colsum_finish_kernel<0>, dim3((F + kFinishCols - 1) / kFinishCols, 1), kFinishCols * kFinishParts, 0, s, partial, P, F, out, nullptr, nullptr, nullptr));
   return SB_OK;
 }
 
