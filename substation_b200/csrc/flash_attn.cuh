@@ -176,6 +176,7 @@ enum { kNoDrop = 0, kPhilox = 1, kAnyMask = 2 };     // masks: none dropped | dr
 struct FwdParams {
   int L, nb;               // sequence length, ceil(L / 128)
   int items;               // units * nb
+  int sweeps;              // 2: a first sweep over the keys finds maximum and sum, so that ALPHA itself is rounded to 16 bits
   int jc, q_swap, k_swap, v_swap;
   float c2;                // scale * log2(e)
   Rng rng;
@@ -192,7 +193,9 @@ struct FwdParams {
 // warps: thread = row, online softmax with a lazily updated reference: exponentials are taken against a maximum that
 // may lag up to 2^8 behind (they stay below 256, exact in every format involved up to the usual relative rounding),
 // and only when some row of a warp exceeds it is the output rescaled.  The masks' generator runs while the tile's
-// scores are still being multiplied.
+// scores are still being multiplied.  With two sweeps the first one only keeps the running maximum and sum.
+// Bound by issue slots (40 % of them the mask generator) and the special-function unit.  B=8, L=512 with masks: 43 us where
+// the scores kernel and the gamma contraction took 62 + 18; B=64, L=256 without: 48 us for 122 + 42.
 template <int MODE>
 __global__ void __launch_bounds__(kFwdThreads, 2)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -249,7 +252,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         load_tile(sq, &tmQ, q_full, p.jc, p.q_swap, j0, u);
       }
       __syncwarp();
-      for (int x = 0; x < 2 * nb; ++x, ++n) {
+      const int first = (p.sweeps - 1) * nb;               // a first sweep reads the keys alone
+      for (int i = 0; i < first + 2 * nb; ++i, ++n) {
+        const int x = i < first ? 2 * i : i - first;       // even: keys of tile x / 2, odd: values
         const uint32_t s = n % kRing, ph = (n / kRing) & 1u;
         ok = __all_sync(0xffffffffu, mbar_wait(kv_empty + 8 * s, ph ^ 1u, 21));
         if (!ok) break;
@@ -266,9 +271,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     uint32_t it = 0, n = 0;
     bool ok = true;
     for (int item = blockIdx.x; item < p.items && ok; item += gridDim.x, ++it) {
-      const uint32_t base = it * 2u * (uint32_t)nb;
-      auto scores = [&](int kb) {
-        const uint32_t x = base + 2u * kb, s = x % kRing;
+      const int first = (p.sweeps - 1) * nb, tiles = first + nb;
+      const uint32_t base = it * (uint32_t)(first + 2 * nb);
+      auto scores = [&](int i) {                           // i-th score tile of the item
+        const uint32_t x = base + (i < first ? i : first + 2 * (i - first)), s = x % kRing;
         ok = __all_sync(0xffffffffu, mbar_wait(kv_full + 8 * s, (x / kRing) & 1u, 22));
         if (!ok) return;
         tc_fence_after();
@@ -276,20 +282,22 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           mma_scores(tmem, sq, ring + s * kTile, p.jc, p.jc);
           umma_commit(s_full);
           umma_commit(kv_empty + 8 * s);
-          if (kb == nb - 1) umma_commit(q_empty);
+          if (i == tiles - 1) umma_commit(q_empty);
         }
         __syncwarp();
       };
       ok = __all_sync(0xffffffffu, mbar_wait(q_full, it & 1u, 22));
       if (!ok) break;
       scores(0);
-      for (int kb = 0; kb < nb && ok; ++kb, ++n) {
+      for (int i = 0; i < tiles && ok; ++i, ++n) {
         ok = __all_sync(0xffffffffu, mbar_wait(p_full, n & 1u, 22));   // the scores have been read, their exponentials written
         if (!ok) break;
         tc_fence_after();
-        if (kb + 1 < nb) scores(kb + 1);
+        if (i + 1 < tiles) scores(i + 1);
         if (!ok) break;
-        const uint32_t x = base + 2u * kb + 1u, s = x % kRing;
+        if (i < first) continue;
+        const int kb = i - first;
+        const uint32_t x = base + first + 2u * kb + 1u, s = x % kRing;
         ok = __all_sync(0xffffffffu, mbar_wait(kv_full + 8 * s, (x / kRing) & 1u, 22));
         if (!ok) break;
         if (kb == 0) {
@@ -311,14 +319,43 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const int rt = q * 32 + lane;
     const uint32_t lanes = (uint32_t)(q * 32) << 16;
     uint8_t* prow = gen + (sp - sq) + rt * 128;
-    uint32_t n = 0;     // key tiles so far
+    uint32_t n = 0, v = 0;     // score tiles and output products so far
     bool ok = true;
     for (int item = blockIdx.x; item < p.items && ok; item += gridDim.x) {
       const int u = item / nb, j = (item % nb) * 128 + rt;
       const bool row = j < L;
       const long long row0 = ((long long)u * L + j) * (long long)L;   // linear index of the row's first score
-      float m = -INFINITY, l = 0.f;
-      for (int kb = 0; kb < nb; ++kb, ++n) {
+      float m = -INFINITY, l = 0.f, ref = 0.f;
+      // first sweep: maximum and sum of the row (scores read twice, nothing written)
+      for (int kb = 0; kb < (p.sweeps - 1) * nb; ++kb, ++n) {
+        const int rem = L - kb * 128;
+        ok = __all_sync(0xffffffffu, mbar_wait(s_full, n & 1u, 23));
+        if (!ok) break;
+        tc_fence_after();
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          uint32_t r[32];
+          tmem_ld32_nowait(tmem + lanes + c * 32, r);
+          attn::tmem_ld_wait32(r);
+          float mx = m;
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            if (c * 32 + e >= rem) r[e] = 0xff800000u;
+            mx = fmaxf(mx, __uint_as_float(r[e]));
+          }
+          const float ms = mx == -INFINITY ? 0.f : mx * p.c2;
+          if (mx > m) l *= attn::ex2_approx((m - mx) * p.c2);
+          m = mx;
+#pragma unroll
+          for (int e = 0; e < 32; ++e) l += attn::ex2_approx(fmaf(__uint_as_float(r[e]), p.c2, -ms));
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_full);
+      }
+      if (!ok) break;
+      if (p.sweeps == 2) ref = (m == -INFINITY ? 0.f : m * p.c2) + log2f(l);
+      for (int kb = 0; kb < nb; ++kb, ++n, ++v) {
         const int rem = L - kb * 128;                                  // columns of this tile inside the row (may exceed 128)
         uint32_t keep[4];
 #pragma unroll
@@ -353,12 +390,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             for (int x = 0; x < 4; ++x) mx4[x] = fmaxf(mx4[x], __uint_as_float(r[e + x]));
         }
         const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-        if (n > 0) {                                   // the previous output multiplication has read its exponentials
-          ok = __all_sync(0xffffffffu, mbar_wait(p_free, (n - 1u) & 1u, 25));
+        if (v > 0) {                                   // the previous output multiplication has read its exponentials
+          ok = __all_sync(0xffffffffu, mbar_wait(p_free, (v - 1u) & 1u, 25));
           if (!ok) break;
           tc_fence_after();
         }
-        if (kb == 0) {
+        if (p.sweeps == 2) {
+        } else if (kb == 0) {
           m = mx;
         } else {
           const bool raise = (mx - m) * p.c2 > kLazy;  // -inf so far: true as soon as a finite score comes
@@ -378,7 +416,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             attn::tmem_st_wait();
           }
         }
-        const float ms = m == -INFINITY ? 0.f : m * p.c2;
+        const float ms = p.sweeps == 2 ? ref : m == -INFINITY ? 0.f : m * p.c2;
         uint32_t ra[32], rb[32];
         tmem_ld32_nowait(tmem + lanes, ra);
         float l0 = 0.f, l1 = 0.f;
@@ -416,14 +454,14 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         chunk(2, ra);
         attn::tmem_ld_wait32(rb);
         chunk(3, rb);
-        l += l0 + l1;
+        if (p.sweeps == 1) l += l0 + l1;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(p_full);
       }
       if (!ok) break;
-      ok = __all_sync(0xffffffffu, mbar_wait(p_free, (n - 1u) & 1u, 25));
+      ok = __all_sync(0xffffffffu, mbar_wait(p_free, (v - 1u) & 1u, 25));
       if (!ok) break;
       tc_fence_after();
       uint32_t r[64];
@@ -435,8 +473,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       __syncwarp();
       if (lane == 0) mbar_arrive(o_empty);
       if (row) {
-        store_cols<64>(p.out + (u / p.B) * p.o_sH + (u % p.B) * p.o_sB + (long long)j * p.o_sRow, p.o_sP, r, 1.f / l);
-        if (p.lse) p.lse[(long long)u * L + j] = (m == -INFINITY ? 0.f : m * p.c2) + log2f(l);
+        store_cols<64>(p.out + (u / p.B) * p.o_sH + (u % p.B) * p.o_sB + (long long)j * p.o_sRow, p.o_sP, r, p.sweeps == 2 ? 1.f : 1.f / l);
+        if (p.lse) p.lse[(long long)u * L + j] = p.sweeps == 2 ? ref : (m == -INFINITY ? 0.f : m * p.c2) + log2f(l);
       }
     }
   }
@@ -493,7 +531,10 @@ struct SlotQueue {
 // columns each), eight element warps (thread = query row, 64 columns) turn them into mask * ALPHA and DBETA in
 // registers, write both to shared memory as 16-bit [j x k] tiles, and these are operands as they lie: K-major
 // for dQ, MN-major for dK and dV.  The next tile's scores are multiplied while this one's are turned; accumulators
-// alternate between two sets so that an item's results are stored while the next item computes.
+// alternate between two sets so that an item's results are stored while the next item computes.  Bound by the element
+// warps: special-function unit (16 exponentials per clock and SM) and the latencies of a tile's hand-overs, 3 700 clocks per
+// tile.  B=8, L=512: 58 us and 5 for the row sums, where scores backward, dX2gamma and dX1QKT+dX2QKT took 41 + 21 + 23;
+// B=96, L=128: 48 + 8 for 37 + 21 + 26; B=2, L=1024: 63 + 4 for eight launches of 160.
 __global__ void __launch_bounds__(kBwdThreads, 1)
 flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmG, const BwdParams p) {

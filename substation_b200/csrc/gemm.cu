@@ -250,7 +250,8 @@ __device__ int g_tc_error = 0;  // first failure code of any tcgen05 kernel on t
 //   kind 2: out2 = C + resid                       (encoder-input gradient)
 //   kind 3: out2 = C + bias, out3 = mask * act(out2)   (bias + activation + dropout)
 //   kind 4: out2 = act'(resid) * mask * C, and its column sums per 32 rows   (dropout + activation backward, bias
-//           gradient); C itself is never stored
+//           gradient); C itself is never stored.  Contraction and separate operator 57 -> 43 + 4 us at B=8, L=512 (58 MB
+//           less traffic), 142 -> 97 + 8 at B=96, L=128
 struct EpiParams {
   int kind;
   int vec_along_m;       // bias indexed by the row (m) instead of the column (n)
@@ -1470,6 +1471,12 @@ int launch_flash_fwd(cudaStream_t s, int H, int B, int L, const void* kqv, long 
       !flash_map(base + 2 * slice, v, units, L, &mv, &p.jc, &p.v_swap, &why))
     return fail(SB_ERR_UNSUPPORTED, "attention, projections: " + why);
   p.L = L; p.nb = (L + 127) / 128; p.items = units * p.nb;
+  // Over few tokens ALPHA is rounded as the separate operators round it (a second look at the keys): with few terms per
+  // parameter gradient, a ReLU whose sign hangs on the rounding of attention moves whole gradient elements (B=2, L=128: the
+  // gradients of a step differed from theirs by 6e-3 to 9e-3 with one sweep, by 2e-3 to 5e-3 with two).  Up to 1024 tokens a
+  // training step waits for the host anyway (290 us, against 130 to 230 us of kernels); inference takes the same path, so
+  // that both have the same bits.
+  p.sweeps = (long long)B * L <= 1024 ? 2 : 1;
   p.c2 = scale * 1.4426950408889634f;
   p.rng = rng;
   p.mask = reinterpret_cast<const uint8_t*>(mask);

@@ -93,10 +93,12 @@ def test_private_passes_with_projections_stored_unit_by_unit():
         assert err <= 8 * HALF[torch.float16], (name, err)
 
 
-def test_row_maxima_that_rise_by_more_than_the_lag():
+@pytest.mark.parametrize('B', [1, 4])
+def test_row_maxima_that_rise_by_more_than_the_lag(B):
     """Scores that grow along the keys by far more than 2^8 per tile: every tile raises the reference maximum and
-    rescales what has been summed so far (std 1.5 projections, keys scaled up with their position)."""
-    dev, B, S, H = torch.device('cuda:0'), 2, 512, 2
+    rescales what has been summed so far (keys scaled up with their position).  512 tokens take two sweeps over the keys,
+    2048 one."""
+    dev, S, H = torch.device('cuda:0'), 512, 2
     E = 64 * H
     enc = Encoder('', B, S, H, E, L.uniform_layouts(), torch.float16, 0., 0., 0., 0., activation='gelu').to(dev)
     ref = Encoder('', B, S, H, E, L.uniform_layouts(), torch.float16, 0., 0., 0., 0., activation='gelu',
