@@ -530,7 +530,10 @@ struct SlotQueue {
 // tiles in memory (4 bytes x 64 x L per key tile) or DBETA itself.  Per tile: scores and dALPHA into tensor memory (128
 // columns each), eight element warps (thread = query row, 64 columns) turn them into mask * ALPHA and DBETA in
 // registers, write both to shared memory as 16-bit [j x k] tiles, and these are operands as they lie: K-major
-// for dQ, MN-major for dK and dV.  The next tile's scores are multiplied while this one's are turned; accumulators
+// for dQ, MN-major for dK and dV.  The next tile's scores are multiplied while this one's are turned, so in dQ items, whose
+// 16-bit tiles alternate, the element warps can be done with tile n + 1 before the MMA warp has looked whether tile n was:
+// two barriers (pd_full) say that a tile is written, n & 1, and neither can run a phase ahead of its waiter, because tile
+// n + 2 needs scores which the MMA warp multiplies only after it has seen tile n.  Accumulators
 // alternate between two sets so that an item's results are stored while the next item computes.  Bound by the element
 // warps: special-function unit (16 exponentials per clock and SM) and the latencies of a tile's hand-overs, 3 700 clocks per
 // tile.  B=8, L=512: 58 us and 5 for the row sums, where scores backward, dX2gamma and dX1QKT+dX2QKT took 41 + 21 + 23;
@@ -543,7 +546,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const uint32_t slots = (raw + 1023u) & ~1023u;
   const uint32_t sds = slots + kSlots * 2 * kTile, spm = sds + 2 * kTile, bars = spm + 2 * kTile;
   const uint32_t full = bars, empty = full + 8 * kSlots, sd_full = empty + 8 * kSlots, sd_empty = sd_full + 8;
-  const uint32_t pd_full = sd_empty + 8, ds_empty = pd_full + 8, acc_full = ds_empty + 16, acc_empty = acc_full + 16;
+  const uint32_t pd_full = sd_empty + 8, ds_empty = pd_full + 16, acc_full = ds_empty + 16, acc_empty = acc_full + 16;
   uint8_t* gen = smem_raw + (slots - raw);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen + (acc_empty + 16 - slots));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -557,8 +560,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     }
     mbar_init(sd_full, 1);
     mbar_init(sd_empty, 8);
-    mbar_init(pd_full, 8);
     for (int i = 0; i < 2; ++i) {
+      mbar_init(pd_full + 8 * i, 8);
       mbar_init(ds_empty + 8 * i, 1);
       mbar_init(acc_full + 8 * i, 1);
       mbar_init(acc_empty + 8 * i, 8);
@@ -620,7 +623,6 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     bool ok = true;
     struct Pending { int item, held, slot; uint32_t it, n; bool first, last; };
     Pending pend{-1, 0, 0, 0u, 0u, false, false};
-    uint32_t npd = 0;
     auto wait_slot = [&](int s) {
       ok = __all_sync(0xffffffffu, mbar_wait(full + 8 * s, (phase >> s) & 1u, 32)) && ok;
       phase ^= 1u << s;
@@ -628,8 +630,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     auto outputs = [&](const Pending& d) {
       const bool qi = is_q(d.item);
       const uint32_t set = d.it % sets;
-      ok = ok && __all_sync(0xffffffffu, mbar_wait(pd_full, npd & 1u, 33));
-      ++npd;
+      ok = ok && __all_sync(0xffffffffu, mbar_wait(pd_full + 8 * (d.n & 1u), (d.n >> 1) & 1u, 33));
       if (ok && d.first) ok = __all_sync(0xffffffffu, mbar_wait(acc_empty + 8 * set, ((d.it / sets) & 1u) ^ 1u, 34));
       if (!ok) return;
       tc_fence_after();
@@ -794,7 +795,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           *reinterpret_cast<uint4*>(dst + ((v ^ (lane & 7)) << 4)) = make_uint4(db[4 * v], db[4 * v + 1], db[4 * v + 2], db[4 * v + 3]);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
-        if (lane == 0) mbar_arrive(pd_full);
+        if (lane == 0) mbar_arrive(pd_full + 8 * (n & 1u));
         if (t == 0 && prev >= 0) finish(prev, it - 1u);
       }
       prev = item;

@@ -83,6 +83,16 @@ def test_private_passes_match_passes_that_keep_everything(B, S, H, dtype, p, mod
         assert err <= 8 * HALF[dtype], (name, err)
 
 
+@pytest.mark.parametrize('B,S,H,mode', [(1, 2048, 4, 'philox'), (3, 1920, 4, 'philox'), (1, 2000, 8, 'explicit')])
+def test_long_streams_of_key_tiles(B, S, H, mode):
+    """dQ items over 15 and 16 key tiles: element warps and product warp hand the two 16-bit tiles over in turn, with nothing
+    but the barriers to keep one from running ahead of the other (a stall would end in the wait limit and be reported)."""
+    kept, private = _passes(B, S, H, torch.float16, 0.1, mode, cases._layouts({'layouts': 'uniform'}), seed=S)
+    for name, want in kept.items():
+        err = ((private[name].double() - want.double()).norm() / want.double().norm()).item()
+        assert err <= 8 * HALF[torch.float16], (name, err)
+
+
 def test_private_passes_with_projections_stored_unit_by_unit():
     """KKQQVV as QHBPJ (the order shipped for B=96, L=128 with the original module)."""
     lay = L.uniform_layouts()
