@@ -414,12 +414,14 @@ __device__ __forceinline__ float act_fwd(float x, int activation) {
 
 __device__ __forceinline__ float act_bwd(float x, float dy, int activation) {
   if (activation == SB_ACT_RELU) return x > 0.f ? dy : 0.f;
-  // d/dx of x * s(x) with s = 1 / (1 + q), q = 2^t as in act_fwd: s + x * s * (1 - s) * 2u', and 1 - s = q * s.
-  // (t is bounded so that q and s stay finite and normal.)
-  const float x2 = x * x;
-  const float q = ex2_unit(fminf(gelu_exponent(x), 126.f));
-  const float s = rcp_unit(1.f + q);
-  return s * fmaf(x * fmaf(x2, 0.21406448f, 1.5957691f), q * s, 1.f) * dy;
+  // d/dx of x * s(x) with s = 1 / (1 + q), q = 2^t as in act_fwd: s + x * s * (1 - s) * 2u', and 1 - s = q * s.  Past
+  // t = 126 (x below -10) s is zero, and x stops at 16 in magnitude, where the derivative is 0 or 1 to the last bit: q, s and
+  // the polynomial stay finite over the whole range of bf16, so that no product of a huge and a tiny factor is left standing.
+  const float xb = fabsf(x) > 16.f ? copysignf(16.f, x) : x;   // (a NaN stays)
+  const float x2 = xb * xb, t = gelu_exponent(xb);
+  const float q = ex2_unit(fminf(t, 126.f));
+  const float s = t > 126.f ? 0.f : rcp_unit(1.f + q);
+  return s * fmaf(xb * fmaf(x2, 0.21406448f, 1.5957691f), q * s, 1.f) * dy;
 }
 
 // Dropout and activation backward of eight packed values: act'(x) * mask * g (ReLU: exact selections of 16-bit values).

@@ -160,6 +160,30 @@ def test_bad_and_bdrlb(B, J, F, lay_in, lay_out, activation):
     assert_close(d_db, db, what='DLINB1')
 
 
+@pytest.mark.parametrize('dtype', [torch.float16, torch.bfloat16])
+def test_gelu_over_every_value_of_the_storage_type(dtype):
+    """Function and derivative at all finite 16-bit values against float64.  Bound: half a unit of the result, and in fp32
+    |t| <= 126 with three roundings behind the exponent and one unit each from ex2 and rcp: s is off by at most
+    s (1 - s) (0.7 * 3 |t| + 4) 2^-24 < 4 * 2^-24, times x (function) or x * 2u' (derivative, < 6 where s (1 - s) counts)."""
+    ops = _ops()
+    x = torch.arange(65536, dtype=torch.int32).to(torch.uint16).view(dtype)
+    x = x[torch.isfinite(x)]
+    x = torch.cat([x, x.new_zeros(-len(x) % 1024)]).view(1, -1, 1024).to(DEV)
+    mask, bias = torch.ones_like(x, dtype=torch.uint8), x.new_zeros(1024)
+    lin1, drop2, dlin1 = (torch.full_like(x, float('nan')) for _ in range(3))
+    ops.bias_activation_dropout(x, bias, mask, lin1, drop2, activation='gelu', p=0.0, mode='explicit')
+    ops.backward_dropout_activation_bias(torch.ones_like(x), mask, lin1, dlin1, bias.clone(), activation='gelu')
+    v = x.double()
+    c = v.clamp(-40, 40)                               # beyond, float64 itself has the limits 0 and 1
+    u = (2 / torch.pi) ** 0.5 * (c + 0.044715 * c ** 3)
+    s, r = torch.sigmoid(2 * u), torch.sigmoid(-2 * u)
+    unit = 2.0 ** (-11 if dtype == torch.float16 else -8)
+    for got, want, lost in ((drop2, v * s, 4 * v.abs().clamp_max(16)),
+                            (dlin1, s + c * s * r * 2 * (2 / torch.pi) ** 0.5 * (1 + 3 * 0.044715 * c * c), 24)):
+        assert torch.isfinite(got).all()
+        assert ((got.double() - want).abs() <= unit * want.abs() + lost * 2.0 ** -24 + 2.0 ** -25).all()
+
+
 @pytest.mark.parametrize('B,J,F,lay', [(4, 64, 1024, 'BJI'), (2, 9, 200, 'BJI'), (2, 16, 128, 'IBJ'),
                                        (3, 8, 520, 'JBI'), (16, 128, 64, 'BJI')])
 def test_token_reductions_bsb_ebsb_baob(B, J, F, lay):
