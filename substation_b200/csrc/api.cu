@@ -1711,24 +1711,43 @@ PrivateScratch private_scratch(const sb_encoder* e, const sb_encoder* t) {
   return PrivateScratch{f.fwd_bytes, f.bwd_bytes, act};
 }
 
-// What a pass of the twin inherits from its handle, and hands back.
-void to_twin(sb_encoder* e, sb_encoder* t) {
-  if (t == e) return;
-  t->fuse = e->fuse; t->dead_stores = e->dead_stores;
-  t->ffn_grads_event = e->ffn_grads_event; t->rewriting = e->rewriting;
-}
-void from_twin(sb_encoder* e, const sb_encoder* t, long long kernels_before, bool forward) {
-  if (t == e) return;
-  e->launches = t->launches;
-  (forward ? e->kernels_fwd : e->kernels_bwd) = g_kernel_launches - kernels_before;
-}
+// A private pass on its target.  A twin inherits its handle's switches and list of timed operators; list, events and counts
+// go back when the pass is over, also when it failed.
+struct TwinPass {
+  sb_encoder *e, *t;
+  const bool forward;
+  const long long k0 = g_kernel_launches;
+  TwinPass(sb_encoder* e, sb_encoder* t, bool forward) : e(e), t(t), forward(forward) {
+    if (t == e) return;
+    t->fuse = e->fuse; t->dead_stores = e->dead_stores; t->timing = e->timing;
+    t->ffn_grads_event = e->ffn_grads_event; t->rewriting = e->rewriting;
+    swap_marks();
+  }
+  ~TwinPass() {
+    if (t == e) return;
+    swap_marks();
+    e->launches = t->launches;
+    (forward ? e->kernels_fwd : e->kernels_bwd) = g_kernel_launches - k0;
+  }
+  void swap_marks() {
+    t->marks.swap(e->marks);
+    t->event_pool.swap(e->event_pool);
+  }
+  TwinPass(const TwinPass&) = delete;
+};
 
-int relayout_x(sb_encoder* from, const void* src, sb_encoder* to, void* dst, cudaStream_t s) {
+// The change of order is timed like an operator but not counted as one (the reference has none such).
+int relayout_x(sb_encoder* from, const void* src, sb_encoder* to, void* dst, cudaStream_t s, sb_encoder* t, bool last) {
   View3 a, b;
+  const int launches = t->launches;
+  t->mark(s, "relayout");
   const sb_tensor ta = from->view(src, TID("X")), tb = to->view(dst, TID("X"));
   SB_TRY(to_view3(&ta, nullptr, false, "relayout.src", &a));
   SB_TRY(to_view3(&tb, &ta, false, "relayout.dst", &b));
-  return launch_relayout(s, dims3(&ta), a, b);
+  SB_TRY(launch_relayout(s, dims3(&ta), a, b));
+  if (last && t->timing) t->mark(s, "");
+  t->launches = launches;
+  return SB_OK;
 }
 
 }  // namespace
@@ -1755,12 +1774,10 @@ extern "C" int sb_encoder_forward_private(sb_encoder* e, void* stream, const voi
   char* acts = reinterpret_cast<char*>(scratch) + ps.attn_fwd;
   const PrivateForward priv{scratch, keep != 0};
   auto pass = [&](cudaStream_t s) {
-    const long long k0 = g_kernel_launches;
-    to_twin(e, t);
-    if (ps.act) SB_TRY(relayout_x(e, x, t, acts, s));
+    const TwinPass on(e, t, true);
+    if (ps.act) SB_TRY(relayout_x(e, x, t, acts, s, t, false));
     SB_TRY(forward_pass(t, (void*)s, ps.act ? acts : x, params, fwd, ps.act ? acts + ps.act : y, mask_mode, seed, offset, &priv));
-    if (ps.act) SB_TRY(relayout_x(t, acts + ps.act, e, y, s));
-    from_twin(e, t, k0, true);
+    if (ps.act) SB_TRY(relayout_x(t, acts + ps.act, e, y, s, t, true));
     return (int)SB_OK;
   };
   return run_pass(e, e->graph_fwd_private, (cudaStream_t)stream, pass);
@@ -1780,13 +1797,11 @@ extern "C" int sb_encoder_backward_private(sb_encoder* e, void* stream, const vo
   char* acts = reinterpret_cast<char*>(scratch) + ps.attn_bwd;
   const PrivateBackward priv{fwd_scratch, scratch};
   auto pass = [&](cudaStream_t s) {
-    const long long k0 = g_kernel_launches;
-    to_twin(e, t);
-    if (ps.act) SB_TRY(relayout_x(e, dy, t, acts, s));
+    const TwinPass on(e, t, false);
+    if (ps.act) SB_TRY(relayout_x(e, dy, t, acts, s, t, false));
     SB_TRY(backward_pass(t, (void*)s, ps.act ? acts : dy, dparams, bwd, params, fwd, ps.act ? xt : x,
                          ps.act ? acts + ps.act : dx, &priv));
-    if (ps.act) SB_TRY(relayout_x(t, acts + ps.act, e, dx, s));
-    from_twin(e, t, k0, false);
+    if (ps.act) SB_TRY(relayout_x(t, acts + ps.act, e, dx, s, t, true));
     return (int)SB_OK;
   };
   return run_pass(e, e->graph_bwd_private, (cudaStream_t)stream, pass);

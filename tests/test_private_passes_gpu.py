@@ -165,3 +165,29 @@ def test_split_k_clusters(M, N, K):
             want = (a.T if am else a).double() @ (b if bm else b.T).double()
             err = ((c.double() - want).norm() / want.norm()).item()
             assert err <= 2.0 ** -11 + K ** 0.5 * 2.0 ** -23, (am, bm, err)
+
+
+@pytest.mark.parametrize('B,S,layouts', [(2, 128, 'uniform'), (3, 77, 'uniform'), (2, 128, 'feature_major')])
+def test_private_passes_are_timed_operator_by_operator(B, S, layouts):
+    """``sb_encoder_set_timing`` covers private passes, also those that run in other orders or with padded rows."""
+    dev, H = torch.device('cuda:0'), 2
+    lay = cases._layouts({'layouts': layouts})
+    enc = Encoder('', B, S, H, 64 * H, lay, torch.float16, 0.1, 0.1, 0.1, 0.1).to(dev)
+    nf, nb = enc.private_arena_bytes(dev)
+    lib = _lib.load()
+    _lib.check(lib.sb_encoder_set_timing(enc._handle, 1), lib)
+    arena, barena, garena = (torch.empty(n, dtype=torch.uint8, device=dev) for n in (nf, nb, enc.arena_bytes('grads')))
+    x = torch.randn(L.shape_of(L.validate(lay)['X'], enc.sizes), device=dev).half()
+    y, dx, weights = torch.empty_like(x), torch.empty_like(x), [p.detach() for p in enc.params]
+    changes = ['relayout'] if layouts == 'feature_major' else []
+    for _ in range(2):
+        enc.forward_private(x, weights, arena, y)
+        assert enc.launch_count() == 7
+        enc.backward_private(y, enc.views('grads', garena), barena, weights, arena, x, dx)
+        names, ms = zip(*enc.op_times())
+        assert all(t > 0 for t in ms)
+        for part in (['QKV-fused+aib', 'attention', 'out', 'bdrln1', 'lin1+bad', 'lin2', 'bdrln2'],
+                     ['bsb+blnrd1', 'attention-backward', 'dWQKV-fused']):
+            assert [n for n in names if n in part] == part, names
+        assert list(names[:1] + names[-1:]) == changes * 2 or not changes and 'relayout' not in names
+        assert names.count('relayout') == 4 * len(changes)
