@@ -764,7 +764,7 @@ bool make_operand_map(const void* ptr, long long R, long long K, long long batch
 
 int g_sm_budget = 0;  // 0: all SMs; otherwise the persistent grid leaves the rest to concurrent kernels
 
-int sm_count() {
+int device_sms() {
   static thread_local int cached_dev = -1, cached = 0;
   int dev = 0;
   cudaGetDevice(&dev);
@@ -772,7 +772,10 @@ int sm_count() {
     cudaDeviceGetAttribute(&cached, cudaDevAttrMultiProcessorCount, dev);
     cached_dev = dev;
   }
-  const int n = cached > 0 ? cached : 148;
+  return cached > 0 ? cached : 148;
+}
+int sm_count() {
+  const int n = device_sms();
   return (g_sm_budget > 0 && g_sm_budget < n) ? g_sm_budget : n;
 }
 
@@ -1053,11 +1056,13 @@ int launch_tc_pair_splitk(cudaStream_t s, const GemmProblem& g, const OperandMap
 // both fit (barriers and remote reads: 10.5 against 6.8 us for `out` at 256 tokens, 15.7 against 12.3 us for dXlin1).
 // Contractions and elementwise operators of an inference pass at 1024 features, together: 40.3 -> 35.4 us at 128 tokens,
 // 58.4 -> 37.0 at 200, 46.4 -> 37.6 at 256; of a training step 104.8 -> 95.5, 135 -> 106, 118.8 -> 105.6 us.
+// The device's SMs count here and not the budget: the number of parts is an order of summation, and results must not
+// depend on the budget.  (Nor does the kernel hold SMs from a collective: its CTAs have one tile each and are gone in 5 to 12 us.)
 int cluster_splits(const GemmProblem& g) {
   if (g.batch != 1 || g.sCn != 1 || std::min(g.M, g.N) > 256 || g.sCm % 8 != 0 || (reinterpret_cast<uintptr_t>(g.C) & 15u))
     return 0;
   const long long tiles = ((g.M + kBM - 1) / kBM) * ((g.N + csk::kBN - 1) / csk::kBN), KT = (g.K + kBK - 1) / kBK;
-  const int sms = sm_count();
+  const int sms = device_sms();
   for (int sk : {4, 2})
     if (tiles * sk <= 2 * sms && KT >= 2 * sk) return sk;
   return 0;
