@@ -1493,7 +1493,8 @@ int launch_flash_fwd(cudaStream_t s, int H, int B, int L, const void* kqv, long 
   auto kernel = none ? flash::flash_fwd_kernel<flash::kNoDrop>
                      : rng.philox && L % 8 == 0 ? flash::flash_fwd_kernel<flash::kPhilox> : flash::flash_fwd_kernel<flash::kAnyMask>;
   SB_CUDA_OK(ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), flash::kFwdSmem));
-  const unsigned grid = (unsigned)std::min<long long>(p.items, 2ll * sm_count());
+  // Two CTAs per SM, but the machine may place one on each SM first: within a budget there is one for every SM of it.
+  const unsigned grid = (unsigned)std::min<long long>(p.items, sm_count() < device_sms() ? sm_count() : 2 * sm_count());
   SB_LAUNCH_OK(launch_k(kernel, grid, flash::kFwdThreads, flash::kFwdSmem, s, mq, mk, mv, p));
   return SB_OK;
 }

@@ -191,3 +191,27 @@ def test_private_passes_are_timed_operator_by_operator(B, S, layouts):
             assert [n for n in names if n in part] == part, names
         assert list(names[:1] + names[-1:]) == changes * 2 or not changes and 'relayout' not in names
         assert names.count('relayout') == 4 * len(changes)
+
+
+def test_attention_forward_stays_within_the_sm_budget(tmp_path):
+    """Two CTAs per SM of the whole device, one per SM of a budget: never on more SMs than the library may use."""
+    import json
+    from substation_b200 import ops
+    dev, B, S, H = torch.device('cuda:0'), 8, 512, 16
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    enc = Encoder('', B, S, H, 64 * H, L.uniform_layouts(), torch.float16, 0.1, 0.1, 0.1, 0.1).to(dev)
+    enc.set_graphs(False)
+    x = torch.randn(B, S, 64 * H, device=dev).half()
+    grids = []
+    try:
+        for budget in (0, 100):
+            ops.set_sm_budget(budget)
+            with torch.no_grad(), torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+                enc(x)
+                torch.cuda.synchronize()
+            path = tmp_path / f'{budget}.json'
+            prof.export_chrome_trace(str(path))
+            grids += [e['args']['grid'][0] for e in json.load(open(path))['traceEvents'] if 'flash_fwd_kernel' in e.get('name', '')]
+    finally:
+        ops.set_sm_budget(0)
+    assert grids == [2 * sms, 100]
