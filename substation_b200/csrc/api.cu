@@ -1696,7 +1696,7 @@ sb_encoder* private_target(sb_encoder* e, int mask_mode) {
 int private_supported(const sb_encoder* e, const sb_encoder* t) {
   if (e->dims[TID("ATTN_DROP_MASK")] != "HBJK" ||
       flash_supported(e->H, e->B, e->S, e->P, proj_view(t->proj), proj_view(t->logical[TID("DGAMMA")])) != SB_OK)
-    return fail(SB_ERR_UNSUPPORTED, "private passes need head size 64, score masks stored as HBJK and projections with unit "
+    return fail(SB_ERR_UNSUPPORTED, "private passes need head size 64, at most 2048 tokens per sample, score masks stored as HBJK and projections with unit "
                                     "stride along the head or the sequence dim");
   return SB_OK;
 }

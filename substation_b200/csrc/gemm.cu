@@ -1435,7 +1435,9 @@ int flash_supported(int H, int B, int L, int P, View4 proj, View4 dgamma) {
     if (v->sH != 1 && v->sK != 1) return SB_ERR_UNSUPPORTED;
     if (v->sH == 1 && (((v->sK | v->sJ | v->sB) & 7) || !unit_view(*v, H, B).collapses)) return SB_ERR_UNSUPPORTED;
   }
-  if (P != 64 || L < 1 || (long long)H * B * ((L + 31) / 32) > 0x3fffffffLL) return SB_ERR_UNSUPPORTED;
+  // (rows beyond 2048 are refused by the operators of a pass that keeps its scores; a pass that is looked at and one that is
+  // not accept the same calls)
+  if (P != 64 || L < 1 || L > 2048 || (long long)H * B * ((L + 31) / 32) > 0x3fffffffLL) return SB_ERR_UNSUPPORTED;
   return SB_OK;
 }
 

@@ -505,7 +505,7 @@ class Encoder(torch.nn.Module):
     def private_arena_bytes(self, device):
         """(forward, backward) arena bytes of passes whose intermediates nobody looks at (``forward_private``), or None
         where such passes do not apply: ``enable_debug``, ``keep_all_intermediates``, ``profiling``, ``fuse=False``,
-        a head size other than 64."""
+        a head size other than 64, samples of more than 2048 tokens."""
         with torch.cuda.device(device):
             plans = self._private_plans(torch.device('cuda', torch.cuda.current_device()))
         return None if plans is None else (plans['fwd'][1], plans['bwd'][1])

@@ -215,3 +215,12 @@ def test_attention_forward_stays_within_the_sm_budget(tmp_path):
     finally:
         ops.set_sm_budget(0)
     assert grids == [2 * sms, 100]
+
+
+@pytest.mark.parametrize('keep', [True, False])
+def test_rows_beyond_2048_are_refused_with_and_without_score_tensors(keep):
+    dev, S = torch.device('cuda:0'), 2056
+    enc = Encoder('', 1, S, 1, 64, L.uniform_layouts(), torch.float16, 0., 0., 0., 0., keep_all_intermediates=keep).to(dev)
+    assert enc.private_arena_bytes(dev) is None
+    with pytest.raises(_lib.SubstationError, match='2048'):
+        enc(torch.zeros(1, S, 64, device=dev).half())
