@@ -520,10 +520,12 @@ class Encoder(torch.nn.Module):
     def forward_private(self, X, weights, arena, Y):
         """One forward pass that keeps what its backward pass needs in ``arena`` (one uint8 tensor of
         ``private_arena_bytes``), in an order of the library's choosing: no score tensors.  Buffers as ``forward_raw``."""
+        return self._forward_private(self._private_plans(X.device), X, weights, arena, Y)
+
+    def _forward_private(self, plans, X, weights, arena, Y):
         self._check_input(X, 'X')
         self._check_input(Y, 'Y')
         self._check_raw(X.device, X=X, Y=Y, weights=list(weights), arena=arena)
-        plans = self._private_plans(X.device)
         if plans is None:
             raise RuntimeError('private passes do not apply to this configuration (see private_arena_bytes)')
         ptrs, scratch = self._private_arena(plans, 'fwd', arena)
@@ -532,12 +534,14 @@ class Encoder(torch.nn.Module):
 
     def backward_private(self, DY, grads, barena, weights, arena, X, DX):
         """The backward pass of ``forward_private``; ``grads``: name -> preallocated tensor."""
+        return self._backward_private(self._private_plans(DY.device), DY, grads, barena, weights, arena, X, DX)
+
+    def _backward_private(self, plans, DY, grads, barena, weights, arena, X, DX):
         self._check_input(DY, 'DY')
         self._check_input(DX, 'DX')
         self._check_input(X, 'X')
         self._check_raw(DY.device, DY=DY, DX=DX, X=X, weights=list(weights), arena=arena, barena=barena,
                         grads={n: grads[n] for n in self._param_names})
-        plans = self._private_plans(DY.device)
         if plans is None:
             raise RuntimeError('private passes do not apply to this configuration (see private_arena_bytes)')
         fptrs, fscratch = self._private_arena(plans, 'fwd', arena)

@@ -3,8 +3,9 @@ data-parallel gradient reduction overlapped with the rest of backward.
 
 The reference times one layer (pytorch_module/run_encoder.py:345-383); a BERT-large
 encoder is 24 of them with independent weights.  Forward keeps what each layer's
-backward needs alive (one arena per layer, allocated once and reused every step; with
-``keep_all_intermediates`` every named intermediate, as views in ``fwd`` and ``bwd``);
+backward needs alive (one arena per layer, allocated once and reused every step; every
+named intermediate, as views in ``fwd`` and ``bwd``, with ``keep_all_intermediates`` or
+once somebody asks for one of the two);
 backward walks the layers in reverse with ONE shared arena for backward
 intermediates, writes layer l's 12 parameter gradients into bucket l and starts
 its sum-allreduce at once, so the reduction of layer l runs beside the backward of
@@ -46,12 +47,15 @@ class EncoderStack:
         # private passes (no score tensors in memory) unless somebody wants to look at the intermediates
         sizes = e0.private_arena_bytes(self.device)
         self.private = sizes is not None
-        nf, nb = sizes or e0.intermediate_bytes()
-        self.arena_bytes = (nf, nb)
-        arenas = [torch.empty(nf, dtype=torch.uint8, device=self.device) for _ in self.layers]
-        barena = torch.empty(nb, dtype=torch.uint8, device=self.device)
-        self.fwd = arenas if self.private else [enc.views('forward', a) for enc, a in zip(self.layers, arenas)]
-        self.bwd = barena if self.private else e0.views('backward', barena)
+        self._named = None                               # (fwd, bwd): views of every intermediate, once they are wanted
+        self._kept = ['nothing'] * num_layers            # how each layer's last forward pass kept what its backward needs
+        self._redo = [None] * num_layers                 # (Philox offset, weight versions) of that pass
+        self._dy0 = None                                 # what layer 0's last backward pass was given
+        if self.private:
+            self._arenas = [torch.empty(sizes[0], dtype=torch.uint8, device=self.device) for _ in self.layers]
+            self._barena = torch.empty(sizes[1], dtype=torch.uint8, device=self.device)
+        else:
+            self._name_intermediates()
         # activations between layers: acts[l] is the input of layer l, acts[-1] the output
         self.acts = [torch.empty(shape_x, dtype=dtype, device=self.device) for _ in range(num_layers + 1)]
         self.dacts = [torch.empty(shape_x, dtype=dtype, device=self.device) for _ in range(2)]
@@ -61,15 +65,67 @@ class EncoderStack:
             raise NotImplementedError('the stack draws its masks in the kernels (Philox); explicit masks are a '
                                       'single-layer testing facility')
 
-    def memory_bytes(self):
+    def _name_intermediates(self):
+        """Buffers for every named intermediate; passes fill them from now on, and what the last passes kept privately is
+        computed again from the activations between the layers (same weights and masks)."""
         e0 = self.layers[0]
-        return len(self.layers) * (self.arena_bytes[0] + e0.arena_bytes('grads')) + self.arena_bytes[1]
+        if self._named is None:
+            self._named = ([enc.views('forward', torch.empty(enc.arena_bytes('forward'), dtype=torch.uint8, device=self.device))
+                            for enc in self.layers],
+                           e0.views('backward', torch.empty(e0.arena_bytes('backward'), dtype=torch.uint8, device=self.device)))
+        again = [l for l, kept in enumerate(self._kept) if kept == 'private']
+        if not again:
+            return
+        fwd, bwd = self._named
+        out = torch.empty_like(self.acts[0])
+        for l in again:
+            enc, (offset, versions) = self.layers[l], self._redo[l]
+            if versions != [w._version for w in self.weights[l]]:
+                raise RuntimeError('the weights changed after the pass whose intermediates are asked for; '
+                                   'build the stack with keep_all_intermediates=True')
+            now, enc.philox_offset = enc.philox_offset, offset
+            enc.forward_raw(self.acts[l], self.weights[l], fwd[l], out)
+            enc.philox_offset = now
+            self._kept[l] = 'named'
+        if self._dy0 is not None and 0 in again:
+            grads = e0.views('grads', torch.empty(e0.arena_bytes('grads'), dtype=torch.uint8, device=self.device))
+            e0.backward_raw(self._dy0, grads, bwd, self.weights[0], fwd[0], self.acts[0], out)
+
+    @property
+    def fwd(self):
+        """Per layer, name -> forward intermediate of the last pass.  Asking makes this and later passes keep them all."""
+        self._name_intermediates()
+        return self._named[0]
+
+    @property
+    def bwd(self):
+        """Name -> backward intermediate of the layer that ran last.  Asking makes this and later passes keep them all."""
+        self._name_intermediates()
+        return self._named[1]
+
+    def memory_bytes(self):
+        e0, n = self.layers[0], len(self.layers)
+        total = n * e0.arena_bytes('grads')
+        if self.private:
+            total += n * self._arenas[0].numel() + self._barena.numel()
+        if self._named is not None:
+            total += n * e0.arena_bytes('forward') + e0.arena_bytes('backward')
+        return total
 
     def forward(self, X):
         self.acts[0].copy_(X)
+        self._dy0 = None
+        self._kept = ['nothing'] * len(self.layers)
         for l, enc in enumerate(self.layers):
-            run = enc.forward_private if self.private else enc.forward_raw
-            run(self.acts[l], self.weights[l], self.fwd[l], self.acts[l + 1])
+            # (a layer whose switches changed since, enable_debug for one, has no private passes any more)
+            plans = enc._private_plans(self.acts[l].device) if self._named is None else None
+            if plans is None:
+                enc.forward_raw(self.acts[l], self.weights[l], self.fwd[l], self.acts[l + 1])
+                self._kept[l] = 'named'
+            else:
+                self._redo[l] = (enc.philox_offset, [w._version for w in self.weights[l]])
+                enc._forward_private(plans, self.acts[l], self.weights[l], self._arenas[l], self.acts[l + 1])
+                self._kept[l] = 'private'
         return self.acts[-1]
 
     def backward(self, DY, trace=None):
@@ -90,8 +146,15 @@ class EncoderStack:
         for l in range(len(self.layers) - 1, -1, -1):
             self.reducer.wait(l)                         # bucket l free again (previous step's reduction done)
             out = self.dacts[l & 1]
-            run = self.layers[l].backward_private if self.private else self.layers[l].backward_raw
-            run(cur, self.grads[l], self.bwd, self.weights[l], self.fwd[l], self.acts[l], out)
+            enc = self.layers[l]
+            plans = enc._private_plans(cur.device) if self._kept[l] == 'private' else None
+            if plans is not None:
+                enc._backward_private(plans, cur, self.grads[l], self._barena, self.weights[l], self._arenas[l],
+                                      self.acts[l], out)
+            else:
+                enc.backward_raw(cur, self.grads[l], self.bwd, self.weights[l], self.fwd[l], self.acts[l], out)
+            if l == 0:
+                self._dy0 = cur
             if tracing:
                 done = torch.cuda.Event(enable_timing=True)
                 done.record()

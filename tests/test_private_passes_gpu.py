@@ -224,3 +224,57 @@ def test_rows_beyond_2048_are_refused_with_and_without_score_tensors(keep):
     assert enc.private_arena_bytes(dev) is None
     with pytest.raises(_lib.SubstationError, match='2048'):
         enc(torch.zeros(1, S, 64, device=dev).half())
+
+
+def _stack(layers):
+    from substation_b200.stack import EncoderStack
+    st = EncoderStack(layers, 2, 128, 2, 128, L.uniform_layouts(), dropout_p=0.1, device='cuda:0', seed=5, activation='gelu',
+                      weight_std=0.1)
+    gen = torch.Generator(device='cuda:0').manual_seed(4)
+    return st, *(torch.randn(2, 128, 128, device='cuda:0', generator=gen).half() for _ in range(2))
+
+
+def test_stack_shows_the_intermediates_of_its_last_pass_when_asked():
+    """``fwd`` and ``bwd`` of a stack hold every named intermediate, also those of a pass that had kept none: same bits as a
+    raw pass over the same input, masks included; later passes keep them as they go."""
+    st, x, dy = _stack(1)
+    enc = st.layers[0]
+    st.forward(x)
+    st.backward(dy)
+    st.wait_gradients()
+    fwd = enc.views('forward', torch.zeros(enc.arena_bytes('forward'), dtype=torch.uint8, device=x.device))
+    bwd = enc.views('backward', torch.zeros(enc.arena_bytes('backward'), dtype=torch.uint8, device=x.device))
+    grads = enc.views('grads', torch.zeros(enc.arena_bytes('grads'), dtype=torch.uint8, device=x.device))
+    dead = ('BETA', 'WKKWQQWVV', 'SB1_LINW1', 'LIN2', 'DATTN_DROP', 'DLN2', 'DLN1', 'DXATT')
+    for step in range(2):
+        enc.philox_offset = 4 * step
+        enc.forward_raw(x, st.weights[0], fwd, torch.empty_like(x))
+        enc.backward_raw(dy, grads, bwd, st.weights[0], fwd, x, torch.empty_like(x))
+        for got, want in ((st.fwd[0], fwd), (st.bwd, bwd)):
+            assert set(got) == set(want)
+            assert all(torch.equal(got[n], want[n]) for n in want if n not in dead + ('__arena__',))
+        assert enc.philox_offset == 4 * step + 4
+        st.forward(x)
+        st.backward(dy)
+        enc.philox_offset = 4 * step + 4
+    st, x, dy = _stack(2)
+    st.forward(x)
+    with torch.no_grad():
+        st.layers[1].params[0].add_(1)
+    with pytest.raises(RuntimeError, match='weights changed'):
+        st.fwd
+
+
+@pytest.mark.parametrize('when', ['before', 'between'])
+def test_stack_runs_on_when_a_layer_is_switched_to_debug(when):
+    st, x, dy = _stack(3)
+    ref, _, _ = _stack(3)
+    y, dx = ref.forward(x), ref.backward(dy)
+    if when == 'before':
+        st.layers[1].enable_debug = True
+    got_y = st.forward(x)
+    st.layers[1].enable_debug = True
+    got_dx = st.backward(dy)
+    st.wait_gradients()
+    for a, b in ((got_y, y), (got_dx, dx), (st.grads[1]['LINB1'], ref.grads[1]['LINB1'])):
+        assert ((a.double() - b.double()).norm() / b.double().norm()).item() <= 3 * 8 * HALF[torch.float16]
