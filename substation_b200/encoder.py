@@ -140,6 +140,18 @@ class _EncoderFunction(torch.autograd.Function):
         return (None, DX, None, None, *grads)
 
 
+class _BoundFunction:
+    """The autograd function of one module, as ``encoder_func.apply(X, anchor, *weights)`` takes it (``anchor``: None, or see
+    ``_EncoderFunction``).  Made on request: a class per module that held the module kept it alive."""
+
+    def __init__(self, outer):
+        self._outer = outer
+
+    def apply(self, X, anchor, *weights):
+        keep = torch.is_grad_enabled() and (anchor is not None or X.requires_grad or any(w.requires_grad for w in weights))
+        return _EncoderFunction.apply(self._outer, X, keep, anchor, *weights)
+
+
 class Encoder(torch.nn.Module):
     """Optimized BERT encoder layer (API of pytorch_module/encoder.py:19-25)."""
 
@@ -681,12 +693,16 @@ class Encoder(torch.nn.Module):
         """Kernels launched by the most recent forward plus the most recent backward."""
         return 0 if self._handle is None else _lib.load(self._lib_key).sb_encoder_kernel_count(self._handle)
 
+    @property
+    def encoder_func(self):
+        """The autograd function under the module (pytorch_module/encoder.py:78-139)."""
+        return _BoundFunction(self)
+
     def forward(self, X):
         """Run the encoder."""
         if self.__dict__.get('_pool_n') and self.__dict__.get('_pool_direct') and torch.is_grad_enabled():
             anchor = self.__dict__.get('_anchor')
             if anchor is None or anchor.device != X.device:
                 anchor = self._anchor = torch.zeros(1, device=X.device, requires_grad=True)
-            return _EncoderFunction.apply(self, X, True, anchor, tuple(p.detach() for p in self.params))
-        keep = torch.is_grad_enabled() and (X.requires_grad or any(p.requires_grad for p in self.params))
-        return _EncoderFunction.apply(self, X, keep, None, *self.params)
+            return self.encoder_func.apply(X, anchor, tuple(p.detach() for p in self.params))
+        return self.encoder_func.apply(X, None, *self.params)

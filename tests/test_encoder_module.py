@@ -99,3 +99,17 @@ def test_pointer_tables_are_remembered_per_arena():
     assert t3 is not t1 and t3[0] == m.data_ptr() and t3[1] == t1[1]
     enc.set_buffer_pool(2)
     assert enc._pooled_ptrs('fwd', plan, a, {}) is not t1
+
+
+def test_encoder_func_is_what_forward_applies():
+    """``encoder_func.apply(X, None, *params)`` is ``forward`` (both end in the check of the input here), and neither it nor
+    anything else keeps a dropped module alive."""
+    import weakref
+    enc = Encoder('', 2, 8, 2, 16, L.uniform_layouts(), torch.float16, 0.1, 0.1, 0.1, 0.1)
+    x = torch.zeros(2, 8, 16, dtype=torch.float16)
+    for call in (enc, lambda t: enc.encoder_func.apply(t, None, *enc.params)):
+        with pytest.raises(ValueError, match='CUDA'):
+            call(x)
+    ref = weakref.ref(enc)
+    del enc, call
+    assert ref() is None
