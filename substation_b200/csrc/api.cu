@@ -731,7 +731,18 @@ struct sb_encoder {
     long long passes = 0, captures = 0, replays = 0;
     void drop() { slot[0].drop(); slot[1].drop(); }
   };
-  GraphCache graph_fwd, graph_bwd, graph_fwd_private, graph_bwd_private;
+  GraphCache graphs_of[6];
+  // Passes that launch other kernels have graphs of their own: the mask mode decides about kernels in all but the backward
+  // pass that keeps its scores.
+  GraphCache& graph_fwd(int mask_mode) { return graphs_of[mask_mode == SB_MASK_PHILOX]; }
+  GraphCache& graph_fwd_private(int mask_mode) { return graphs_of[2 + (mask_mode == SB_MASK_PHILOX)]; }
+  GraphCache& graph_bwd_private(int mask_mode) { return graphs_of[4 + (mask_mode == SB_MASK_PHILOX)]; }
+  GraphCache graph_bwd;
+  void drop_backward_graphs() {
+    graph_bwd.drop();
+    graphs_of[4].drop();
+    graphs_of[5].drop();
+  }
   // The same layer with every intermediate in its logical order (parameters as configured): what private passes run
   // when some activation of this configuration does not have its features innermost, or the token count is off the 8 grid.
   std::unique_ptr<sb_encoder> twin;
@@ -1052,10 +1063,8 @@ extern "C" int sb_encoder_destroy(sb_encoder* e) {
   for (auto& m : e->marks) cudaEventDestroy(m.second);
   for (auto ev : e->event_pool) cudaEventDestroy(ev);
   if (e->workspace) cudaFree(e->workspace);
-  e->graph_fwd.drop();
-  e->graph_bwd.drop();
-  e->graph_fwd_private.drop();
-  e->graph_bwd_private.drop();
+  e->drop_backward_graphs();
+  for (auto& c : e->graphs_of) c.drop();
   if (e->capture_stream) cudaStreamDestroy(e->capture_stream);
   delete e;
   return SB_OK;
@@ -1090,20 +1099,18 @@ extern "C" int sb_encoder_set_graphs(sb_encoder* e, int enabled) {
 extern "C" int sb_encoder_set_ffn_grads_event(sb_encoder* e, void* event) {
   if (!e) return fail(SB_ERR_ARG, "null handle");
   // graphs captured so far record the previous event (or none)
-  if (e->ffn_grads_event != (cudaEvent_t)event) {
-    e->graph_bwd.drop();
-    e->graph_bwd_private.drop();
-  }
+  if (e->ffn_grads_event != (cudaEvent_t)event) e->drop_backward_graphs();
   e->ffn_grads_event = (cudaEvent_t)event;
   return SB_OK;
 }
 
 extern "C" int sb_encoder_graph_stats(sb_encoder* e, long long* captures, long long* replays) {
   if (!e || !captures || !replays) return fail(SB_ERR_ARG, "sb_encoder_graph_stats: null argument");
-  *captures = *replays = 0;
-  for (const auto* c : {&e->graph_fwd, &e->graph_bwd, &e->graph_fwd_private, &e->graph_bwd_private}) {
-    *captures += c->captures;
-    *replays += c->replays;
+  *captures = e->graph_bwd.captures;
+  *replays = e->graph_bwd.replays;
+  for (const auto& c : e->graphs_of) {
+    *captures += c.captures;
+    *replays += c.replays;
   }
   return SB_OK;
 }
@@ -1635,7 +1642,10 @@ int run_pass(sb_encoder* e, sb_encoder::GraphCache& cache, cudaStream_t s, Pass&
       SB_CUDA_OK(cudaGraphLaunch(g.exec, s));
       return SB_OK;
     }
-    g.drop();   // other kernels than before (a switch of the handle, another SM budget): capture again
+    // Other kernels than before (a switch of the handle, a misaligned buffer): capture again, but a program that changes
+    // between them all the time pays for one capture in eight graph launches at most and gets plain launches otherwise.
+    if (cache.captures * 8 > cache.replays + 32) return pass(s);
+    g.drop();
   }
   if (!e->capture_stream && cudaStreamCreateWithFlags(&e->capture_stream, cudaStreamNonBlocking) != cudaSuccess) {
     cudaGetLastError();
@@ -1670,7 +1680,7 @@ extern "C" int sb_encoder_forward(sb_encoder* e, void* stream, const void* x, co
                                   void* const* fwd, void* y, int mask_mode, uint64_t seed, uint64_t offset) {
   if (!e || !y || !params || !fwd) return fail(SB_ERR_ARG, "sb_encoder_forward: null argument");
   auto pass = [&](cudaStream_t s) { return forward_pass(e, (void*)s, x, params, fwd, y, mask_mode, seed, offset, nullptr); };
-  return run_pass(e, e->graph_fwd, (cudaStream_t)stream, pass);
+  return run_pass(e, e->graph_fwd(mask_mode), (cudaStream_t)stream, pass);
 }
 
 extern "C" int sb_encoder_backward(sb_encoder* e, void* stream, const void* dy, void* const* dparams,
@@ -1780,7 +1790,7 @@ extern "C" int sb_encoder_forward_private(sb_encoder* e, void* stream, const voi
     if (ps.act) SB_TRY(relayout_x(t, acts + ps.act, e, y, s, t, true));
     return (int)SB_OK;
   };
-  return run_pass(e, e->graph_fwd_private, (cudaStream_t)stream, pass);
+  return run_pass(e, e->graph_fwd_private(mask_mode), (cudaStream_t)stream, pass);
 }
 
 extern "C" int sb_encoder_backward_private(sb_encoder* e, void* stream, const void* dy, void* const* dparams,
@@ -1804,5 +1814,5 @@ extern "C" int sb_encoder_backward_private(sb_encoder* e, void* stream, const vo
     if (ps.act) SB_TRY(relayout_x(t, acts + ps.act, e, dx, s, t, true));
     return (int)SB_OK;
   };
-  return run_pass(e, e->graph_bwd_private, (cudaStream_t)stream, pass);
+  return run_pass(e, e->graph_bwd_private(mask_mode), (cudaStream_t)stream, pass);
 }
