@@ -8,6 +8,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -690,6 +691,9 @@ bool is_permutation(const std::string& a, const std::string& b) {
 }  // namespace
 
 struct sb_encoder {
+  // A pass writes its pointers into the contractions planned once and rewrites the parameters of captured graphs: calls on one
+  // handle from several threads take turns.
+  std::mutex mutex;
   int B, S, H, P, I, U;
   int activation;
   float p_softmax, p_resid1, p_act, p_resid2;
@@ -1072,6 +1076,7 @@ extern "C" int sb_encoder_destroy(sb_encoder* e) {
 
 extern "C" int sb_encoder_set_timing(sb_encoder* e, int enabled) {
   if (!e) return fail(SB_ERR_ARG, "null handle");
+  const std::lock_guard<std::mutex> turn(e->mutex);
   e->timing = enabled != 0;
   return SB_OK;
 }
@@ -1080,24 +1085,28 @@ extern "C" int sb_encoder_launch_count(sb_encoder* e) { return e ? e->launches :
 extern "C" int sb_encoder_kernel_count(sb_encoder* e) { return e ? (int)(e->kernels_fwd + e->kernels_bwd) : 0; }
 extern "C" int sb_encoder_set_fusion(sb_encoder* e, int enabled) {
   if (!e) return fail(SB_ERR_ARG, "null handle");
+  const std::lock_guard<std::mutex> turn(e->mutex);
   e->fuse = enabled != 0;
   return SB_OK;
 }
 
 extern "C" int sb_encoder_set_dead_stores(sb_encoder* e, int enabled) {
   if (!e) return fail(SB_ERR_ARG, "null handle");
+  const std::lock_guard<std::mutex> turn(e->mutex);
   e->dead_stores = enabled != 0;
   return SB_OK;
 }
 
 extern "C" int sb_encoder_set_graphs(sb_encoder* e, int enabled) {
   if (!e) return fail(SB_ERR_ARG, "null handle");
+  const std::lock_guard<std::mutex> turn(e->mutex);
   e->graphs = enabled != 0;
   return SB_OK;
 }
 
 extern "C" int sb_encoder_set_ffn_grads_event(sb_encoder* e, void* event) {
   if (!e) return fail(SB_ERR_ARG, "null handle");
+  const std::lock_guard<std::mutex> turn(e->mutex);
   // graphs captured so far record the previous event (or none)
   if (e->ffn_grads_event != (cudaEvent_t)event) e->drop_backward_graphs();
   e->ffn_grads_event = (cudaEvent_t)event;
@@ -1106,6 +1115,7 @@ extern "C" int sb_encoder_set_ffn_grads_event(sb_encoder* e, void* event) {
 
 extern "C" int sb_encoder_graph_stats(sb_encoder* e, long long* captures, long long* replays) {
   if (!e || !captures || !replays) return fail(SB_ERR_ARG, "sb_encoder_graph_stats: null argument");
+  const std::lock_guard<std::mutex> turn(e->mutex);
   *captures = e->graph_bwd.captures;
   *replays = e->graph_bwd.replays;
   for (const auto& c : e->graphs_of) {
@@ -1117,6 +1127,7 @@ extern "C" int sb_encoder_graph_stats(sb_encoder* e, long long* captures, long l
 
 extern "C" int sb_encoder_get_timing(sb_encoder* e, int max, const char** names, float* ms) {
   if (!e) return 0;
+  const std::lock_guard<std::mutex> turn(e->mutex);
   if (!e->marks.empty()) {
     // marks: begin-of-op events plus one closing event named "" per pass
     cudaEventSynchronize(e->marks.back().second);
@@ -1679,6 +1690,7 @@ int run_pass(sb_encoder* e, sb_encoder::GraphCache& cache, cudaStream_t s, Pass&
 extern "C" int sb_encoder_forward(sb_encoder* e, void* stream, const void* x, const void* const* params,
                                   void* const* fwd, void* y, int mask_mode, uint64_t seed, uint64_t offset) {
   if (!e || !y || !params || !fwd) return fail(SB_ERR_ARG, "sb_encoder_forward: null argument");
+  const std::lock_guard<std::mutex> turn(e->mutex);
   auto pass = [&](cudaStream_t s) { return forward_pass(e, (void*)s, x, params, fwd, y, mask_mode, seed, offset, nullptr); };
   return run_pass(e, e->graph_fwd(mask_mode), (cudaStream_t)stream, pass);
 }
@@ -1688,6 +1700,7 @@ extern "C" int sb_encoder_backward(sb_encoder* e, void* stream, const void* dy, 
                                    const void* x, void* dx) {
   if (!e || !dy || !dparams || !bwd || !dx || !params || !fwd)
     return fail(SB_ERR_ARG, "sb_encoder_backward: null argument");
+  const std::lock_guard<std::mutex> turn(e->mutex);
   auto pass = [&](cudaStream_t s) { return backward_pass(e, (void*)s, dy, dparams, bwd, params, fwd, x, dx, nullptr); };
   return run_pass(e, e->graph_bwd, (cudaStream_t)stream, pass);
 }
@@ -1764,6 +1777,7 @@ int relayout_x(sb_encoder* from, const void* src, sb_encoder* to, void* dst, cud
 
 extern "C" int sb_encoder_private_bytes(sb_encoder* e, int mask_mode, size_t* forward, size_t* backward) {
   if (!e || !forward || !backward) return fail(SB_ERR_ARG, "sb_encoder_private_bytes: null argument");
+  const std::lock_guard<std::mutex> turn(e->mutex);
   *forward = *backward = 0;
   const sb_encoder* t = private_target(e, mask_mode);
   if (!e->fuse || e->dead_stores || private_supported(e, t) != SB_OK) return SB_OK;
@@ -1778,6 +1792,7 @@ extern "C" int sb_encoder_forward_private(sb_encoder* e, void* stream, const voi
                                           uint64_t seed, uint64_t offset) {
   if (!e || !x || !y || !params || !fwd || !scratch) return fail(SB_ERR_ARG, "sb_encoder_forward_private: null argument");
   if (!aligned(scratch, 16)) return fail(SB_ERR_ALIGNMENT, "sb_encoder_forward_private: scratch is not 16-byte aligned");
+  const std::lock_guard<std::mutex> turn(e->mutex);
   sb_encoder* t = private_target(e, mask_mode);
   SB_TRY(private_supported(e, t));
   const PrivateScratch ps = private_scratch(e, t);
@@ -1800,6 +1815,7 @@ extern "C" int sb_encoder_backward_private(sb_encoder* e, void* stream, const vo
     return fail(SB_ERR_ARG, "sb_encoder_backward_private: null argument");
   if (!aligned(fwd_scratch, 16) || !aligned(scratch, 16))
     return fail(SB_ERR_ALIGNMENT, "sb_encoder_backward_private: scratch is not 16-byte aligned");
+  const std::lock_guard<std::mutex> turn(e->mutex);
   sb_encoder* t = private_target(e, mask_mode);
   SB_TRY(private_supported(e, t));
   const PrivateScratch ps = private_scratch(e, t);

@@ -98,3 +98,30 @@ def test_passes_that_keep_changing_their_kernels_are_not_captured_each_time():
         assert torch.equal(*got), step
     captures, replays = encs[0].graph_stats()
     assert replays > 0 and captures <= 5 + steps // 8
+
+
+def test_one_module_used_by_two_threads():
+    """Host calls on one handle take turns: inference from two threads, a stream each, gives what it gives one by one.
+    (128 tokens: no operator of these passes uses the handle's workspaces.)"""
+    import threading
+    dev = torch.device('cuda:0')
+    enc = Encoder('', 1, 128, 2, 128, L.uniform_layouts(), torch.float16, 0., 0., 0., 0.).to(dev)
+    gen = torch.Generator(device=dev).manual_seed(9)
+    xs = [[torch.randn(1, 128, 128, device=dev, generator=gen).half() for _ in range(100)] for _ in range(2)]
+    with torch.no_grad():
+        want = [[enc(x) for x in part] for part in xs]
+    torch.cuda.synchronize()
+    got = [[], []]
+
+    def work(i):
+        with torch.no_grad(), torch.cuda.stream(torch.cuda.Stream(dev)):
+            got[i] += [enc(x) for x in xs[i]]
+            torch.cuda.current_stream().synchronize()
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for part, ref in zip(got, want):
+        assert len(part) == len(ref) and all(torch.equal(a, b) for a, b in zip(part, ref))
+    assert ops.device_error() == 0
