@@ -27,6 +27,18 @@ def get_layouts(which):
     return L.named_layouts(which)
 
 
+def uniform_or_feature_major(which):
+    """'uniform', or 'feature_major': the activations' dim orders of the configuration shipped for B=8, L=512 (most of them
+    feature-major), everything else as in the uniform one."""
+    lay = L.uniform_layouts()
+    if which == 'feature_major':
+        shipped = L.validate(get_layouts('b8_l512'))
+        for key in ('params', 'forward_interm', 'backward_interm'):
+            lay[key] = [(n, shipped[n] if L.LOGICAL[n].startswith('BJ') else dims) for n, dims in lay[key]]
+        lay['input'], lay['output'] = ('X', shipped['X']), ('SB2', shipped['SB2'])
+    return lay
+
+
 def to_dev(a, logical, layout, device, dtype=torch.float16):
     return torch.from_numpy(orc.to_layout(np.asarray(a), logical, layout)).to(device=device, dtype=dtype)
 
@@ -135,3 +147,52 @@ def run_layer_case(B, J, H, P, layouts='uniform', p=0.1, activation='relu', mask
         assert ag is not None and np.array_equal(ag.float().cpu().numpy(), enc.debug['D' + n].astype(np.float32)), n
     worst = max(report.values())
     return (worst, report) if return_report else worst
+
+
+def run_private_case(B, J, H, layouts='uniform', p=0.1, activation='relu', mask_mode='philox', seed=0, tol=1e-2,
+                     dtype=torch.float16, case=None):
+    """The path a user gets by default (autograd, nobody looks at the intermediates) against the oracle: output, input
+    gradient and twelve parameter gradients.  With ReLU the oracle's backward takes the pass's own activation pattern, from
+    the module's buffers and under the checks of ``run_layer_case``.  Returns the module and its pass's DLIN1 (float64)."""
+    device, P = 'cuda:0', 64
+    lay = uniform_or_feature_major(layouts)
+    table, I, U = L.validate(lay), H * P, 4 * H * P
+    X, DY, params, masks = case or make_case(B, J, H, P, seed, (p,) * 4, explicit_masks=mask_mode == 'explicit', dtype=dtype)
+    enc = Encoder('', B, J, H, I, lay, dtype, p, p, p, p, activation=activation, mask_mode=mask_mode, seed=seed).to(device)
+    with torch.no_grad():
+        for (name, layout), prm in zip(lay['params'], enc.params):
+            prm.copy_(to_dev(params[name], L.LOGICAL[name], layout, device, dtype))
+    if mask_mode == 'explicit':
+        enc.set_masks({n: to_dev(masks[n], L.LOGICAL[n], table[n], device, torch.uint8) for n in L.MASKS})
+    else:
+        shapes = {'ATTN_DROP_MASK': (H, B, J, J), 'DROP2MASK': (B, J, U)}
+        masks = {n: orc.philox_mask(shapes.get(n, (B, J, I)), p, seed, site) for site, n in enumerate(L.MASKS)}
+    enc.set_buffer_pool(1, direct_grads=False)           # the pass's buffers stay at hand
+    x = to_dev(X, 'BJI', table['X'], device, dtype).requires_grad_(True)
+    y = enc(x)
+    y.backward(to_dev(DY, 'BJI', table['SB2'], device, dtype))
+    torch.cuda.synchronize()
+    plans = enc._private_plans(x.device)
+    assert plans is not None, 'this configuration has no private passes'
+
+    def kept(which, name):                               # (in logical order, whatever the configuration says)
+        for n, _, _, off, nbytes in plans[which][0]:
+            if n == name:
+                return enc._pool[0][which][off:off + nbytes].view(dtype).view(B, J, U).double().cpu().numpy()
+    f = orc.encoder_forward(X, params, masks, activation=activation)
+    pattern = None
+    if activation == 'relu':
+        pattern = kept('fwd', 'LIN1') > 0
+        differs = pattern != (f['LIN1'] > 0)
+        near = 4e-3 if dtype == torch.float16 else 3.2e-2
+        assert (np.abs(f['LIN1'][differs]) < near * max(1.0, float(np.sqrt((f['LIN1'] ** 2).mean())))).all()
+        assert differs.mean() < (5e-3 if dtype == torch.float16 else 4e-2)
+    g = orc.encoder_backward(X, DY, params, f, activation=activation, relu_pattern=pattern)
+    pairs = [('Y', y, table['SB2'], f['SB2']), ('DX', x.grad, table['X'], g['DX'])]
+    pairs += [('D' + n, getattr(enc, n).grad, table[n], g['D' + n]) for n in enc._param_names]
+    for name, got, layout, want in pairs:
+        got = orc.from_layout(got.detach().double().cpu().numpy(), layout, L.LOGICAL.get(name[1:], 'BJI') if name[0] == 'D' and name != 'DX' else 'BJI')
+        assert np.isfinite(got).all(), name
+        r = orc.rel_l2(got, want)
+        assert r <= tol, f'{name}: rel-L2 {r:.3e} > {tol}'
+    return enc, kept('bwd', 'DLIN1')

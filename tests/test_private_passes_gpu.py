@@ -12,7 +12,7 @@ import pytest
 import torch
 
 from substation_b200 import Encoder, layouts as L, _lib
-from perf import cases
+from tests.layer_harness import run_private_case, uniform_or_feature_major
 
 pytestmark = pytest.mark.gpu
 HALF = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}
@@ -75,7 +75,7 @@ def _passes(B, S, H, dtype, p, mode, lay, seed, activation='gelu'):
     (2, 256, 4, torch.float16, 0.1, 'explicit', 'feature_major'),    # the caller's masks keep their order
 ])
 def test_private_passes_match_passes_that_keep_everything(B, S, H, dtype, p, mode, layouts):
-    kept, private = _passes(B, S, H, dtype, p, mode, cases._layouts({'layouts': layouts}), seed=B * 1000 + S)
+    kept, private = _passes(B, S, H, dtype, p, mode, uniform_or_feature_major(layouts), seed=B * 1000 + S)
     for name, want in kept.items():
         got = private[name]
         assert torch.isfinite(got).all(), name
@@ -87,10 +87,35 @@ def test_private_passes_match_passes_that_keep_everything(B, S, H, dtype, p, mod
 def test_long_streams_of_key_tiles(B, S, H, mode):
     """dQ items over 15 and 16 key tiles: element warps and product warp hand the two 16-bit tiles over in turn, with nothing
     but the barriers to keep one from running ahead of the other (a stall would end in the wait limit and be reported)."""
-    kept, private = _passes(B, S, H, torch.float16, 0.1, mode, cases._layouts({'layouts': 'uniform'}), seed=S)
+    kept, private = _passes(B, S, H, torch.float16, 0.1, mode, L.uniform_layouts(), seed=S)
     for name, want in kept.items():
         err = ((private[name].double() - want.double()).norm() / want.double().norm()).item()
         assert err <= 8 * HALF[torch.float16], (name, err)
+
+
+@pytest.mark.parametrize('B,S,H,dtype,activation,mode,layouts', [
+    (2, 128, 4, torch.float16, 'relu', 'philox', 'uniform'),         # split-K clusters with bias, activation, dropout
+    (1, 77, 8, torch.float16, 'gelu', 'explicit', 'uniform'),
+    (2, 64, 4, torch.bfloat16, 'relu', 'explicit', 'uniform'),
+    (16, 77, 8, torch.float16, 'relu', 'philox', 'uniform'),         # the activation's backward in dXlin2's epilogue over
+    (16, 77, 8, torch.bfloat16, 'relu', 'philox', 'uniform'),        # 1232 tokens: a last tile with 208 of 256 rows, the
+    (16, 77, 8, torch.float16, 'gelu', 'explicit', 'uniform'),       # last block of 32 with 16
+    (12, 200, 12, torch.bfloat16, 'gelu', 'philox', 'uniform'),
+    (5, 100, 16, torch.float16, 'relu', 'philox', 'feature_major'),  # other orders and padded rows
+    (4, 512, 16, torch.float16, 'relu', 'explicit', 'uniform'),
+])
+def test_default_path_against_the_oracle(B, S, H, dtype, activation, mode, layouts):
+    enc, dlin1 = run_private_case(B, S, H, layouts=layouts, activation=activation, mask_mode=mode, seed=S, dtype=dtype,
+                                  tol=1e-2 if dtype == torch.float16 else 5e-2)
+    # LINB1's gradient is the column sums of DLIN1 as stored: fp32 sums, one rounding to 16 bits
+    got, want = enc.LINB1.grad.double().cpu(), torch.from_numpy(dlin1).sum((0, 1))
+    assert ((got - want).norm() / want.norm()).item() <= HALF[dtype] + 1e-5
+    lib = _lib.load(_lib.dtype_key(dtype))
+    _lib.check(lib.sb_encoder_set_timing(enc._handle, 1), lib)
+    x = torch.zeros(L.shape_of(enc._table['X'], enc.sizes), device='cuda:0', dtype=dtype, requires_grad=True)
+    enc(x).sum().backward()
+    names = [n for n, _ in enc.op_times()]
+    assert ('dXlin2+bdrlb' in names) == (B * S >= 1232), names
 
 
 def test_private_passes_with_projections_stored_unit_by_unit():
@@ -142,7 +167,7 @@ def test_row_maxima_that_rise_by_more_than_the_lag(B):
 ])
 def test_token_counts_off_the_vector_grid(B, S, H, dtype, mode):
     for layouts in ('uniform', 'feature_major'):
-        kept, private = _passes(B, S, H, dtype, 0.1, mode, cases._layouts({'layouts': layouts}), seed=S)
+        kept, private = _passes(B, S, H, dtype, 0.1, mode, uniform_or_feature_major(layouts), seed=S)
         for name, want in kept.items():
             err = ((private[name].double() - want.double()).norm() / want.double().norm()).item()
             assert torch.isfinite(private[name]).all() and err <= 8 * HALF[dtype], (layouts, name, err)
@@ -171,7 +196,7 @@ def test_split_k_clusters(M, N, K):
 def test_private_passes_are_timed_operator_by_operator(B, S, layouts):
     """``sb_encoder_set_timing`` covers private passes, also those that run in other orders or with padded rows."""
     dev, H = torch.device('cuda:0'), 2
-    lay = cases._layouts({'layouts': layouts})
+    lay = uniform_or_feature_major(layouts)
     enc = Encoder('', B, S, H, 64 * H, lay, torch.float16, 0.1, 0.1, 0.1, 0.1).to(dev)
     nf, nb = enc.private_arena_bytes(dev)
     lib = _lib.load()
