@@ -12,7 +12,7 @@ and the layer's 12 parameter gradients are sum-allreduced over NCCL, overlapped
 with the next step.  Rank 0 prints ONE JSON line.
 
 value        sequences/s over all ranks, inputs resident in HBM, CUDA-event timed
-e2e          same through the public ``Encoder`` module with host buffers:
+e2e          same through the public ``Encoder`` module on its default path with host buffers:
              pinned-host X and dY copied in, Y and dX copied out, every step;
              copy_only_ms_per_step = the same copies with no compute
 sustained    the same step repeated for at least two seconds, with the SM clock
@@ -733,9 +733,12 @@ def run_ours(args):
         works = [None, None]
         for prm in enc.params:
             prm.requires_grad_(True)
-        # The module keeps two sets of buffers for its autograd path and uses them in turn (set_buffer_pool): the
-        # pointers of a pass repeat every other step, so passes replay as CUDA graphs, and the collective sees the
-        # same two gradient buckets every step.  Y and dX are copied to the host before their set comes round again.
+        # The module as a program that trains has it: with profiling it would run the passes whose operators the table
+        # above lists, which store every intermediate, instead of its default ones.
+        enc.profiling = False
+        # The module keeps two sets of buffers for its autograd path and uses them in turn (set_buffer_pool): nothing
+        # is allocated per pass, and the collective sees the same two gradient buckets every step.  Y and dX are copied to
+        # the host before their set comes round again.
         enc.set_buffer_pool(2)
 
         def copy_in(i):
