@@ -195,7 +195,7 @@ def test_split_k_clusters(M, N, K):
 @pytest.mark.parametrize('B,S,layouts', [(2, 128, 'uniform'), (3, 77, 'uniform'), (2, 128, 'feature_major')])
 def test_private_passes_are_timed_operator_by_operator(B, S, layouts):
     """``sb_encoder_set_timing`` covers private passes, also those that run in other orders or with padded rows."""
-    dev, H = torch.device('cuda:0'), 2
+    dev, H = torch.device('cuda:0'), 8                       # wide enough for the fused contractions of few tokens
     lay = uniform_or_feature_major(layouts)
     enc = Encoder('', B, S, H, 64 * H, lay, torch.float16, 0.1, 0.1, 0.1, 0.1).to(dev)
     nf, nb = enc.private_arena_bytes(dev)
