@@ -1242,7 +1242,7 @@ static int forward_pass(sb_encoder* e, void* stream, const void* x, const void* 
     SB_TRY(to_rng(&d, &rng));
     SB_TRY(launch_flash_fwd(s, e->H, e->B, e->S, T[TID("KKQQVV")], slice, proj_view(e->proj), T[TID("GAMMA")],
                             proj_view(e->logical[TID("GAMMA")]), T[TID("ATTN_DROP_MASK")], 1.f / std::sqrt((float)e->P), rng,
-                            priv->scratch, priv->keep));
+                            priv->scratch, priv->keep, e->activation == SB_ACT_RELU));
   }
   // F2 + softmax.  K and V views are the J-indexed projections relabelled with K.
   if (!priv) {

@@ -1451,7 +1451,7 @@ void flash_scratch(int H, int B, int L, bool pad_proj, bool pad_dgamma, FlashScr
 }
 
 int launch_flash_fwd(cudaStream_t s, int H, int B, int L, const void* kqv, long long slice, View4 proj, void* gamma, View4 gv,
-                     const void* mask, float scale, Rng rng, void* scratch, bool keep) {
+                     const void* mask, float scale, Rng rng, void* scratch, bool keep, bool relu) {
   std::call_once(g_encode_once, load_encode);
   if (!g_encode) return fail(SB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   const int units = H * B;
@@ -1478,12 +1478,14 @@ int launch_flash_fwd(cudaStream_t s, int H, int B, int L, const void* kqv, long 
       !flash_map(base + 2 * slice, v, units, L, &mv, &p.jc, &p.v_swap, &why))
     return fail(SB_ERR_UNSUPPORTED, "attention, projections: " + why);
   p.L = L; p.nb = (L + 127) / 128; p.items = units * p.nb;
-  // Over few tokens ALPHA is rounded as the separate operators round it (a second look at the keys): with few terms per
-  // parameter gradient, a ReLU whose sign hangs on the rounding of attention moves whole gradient elements (B=2, L=128: the
-  // gradients of a step differed from theirs by 6e-3 to 9e-3 with one sweep, by 2e-3 to 5e-3 with two).  Up to 1024 tokens a
-  // training step waits for the host anyway (290 us, against 130 to 230 us of kernels); inference takes the same path, so
-  // that both have the same bits.
-  p.sweeps = (long long)B * L <= 1024 ? 2 : 1;
+  // ReLU layers over few tokens round ALPHA as passes that keep it do, at the price of a second look at the keys (0.5 to 1 us).
+  // This is agreement with those passes and not accuracy: against float64 both forms are alike (Y, DX and the gradients of
+  // WO, WKQV and LINW1, means over ten seeds at 16 to 1024 tokens: 0.95 to 1.20 of one sweep's error in ReLU layers, 1.00 to
+  // 1.04 with GELU).  But where ReLU's sign hangs on how attention rounded, whole elements of a gradient move, and few tokens
+  // do not average them out: at B=2, L=128 a step's gradients are within 6e-3 of a keeping pass with two sweeps and
+  // within 1e-2 with one, single elements 0.9 and 1.1 times the root mean square apart; at 1024 tokens 0.36 and 0.53.  GELU
+  // has no such step.  With and without gradients the form is the same, so that both have the same bits.
+  p.sweeps = relu && (long long)B * L <= 1024 ? 2 : 1;
   p.c2 = scale * 1.4426950408889634f;
   p.rng = rng;
   p.mask = reinterpret_cast<const uint8_t*>(mask);

@@ -86,7 +86,7 @@ int flash_supported(int H, int B, int L, int P, View4 proj, View4 dgamma);
 bool flash_padded(const View4& v, int H, int B, int L);
 void flash_scratch(int H, int B, int L, bool pad_proj, bool pad_dgamma, FlashScratch* f);
 int launch_flash_fwd(cudaStream_t s, int H, int B, int L, const void* kqv, long long slice, View4 proj, void* gamma, View4 gv,
-                     const void* mask, float scale, Rng rng, void* scratch, bool keep);
+                     const void* mask, float scale, Rng rng, void* scratch, bool keep, bool relu);
 int launch_flash_bwd(cudaStream_t s, int H, int B, int L, const void* kqv, long long slice, View4 proj, const void* gamma, View4 gv,
                      const void* dgamma, View4 dgv, void* dkqv, long long dslice, View4 dproj, float scale, const void* fwd_scratch,
                      void* bwd_scratch);

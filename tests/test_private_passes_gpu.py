@@ -103,6 +103,9 @@ def test_long_streams_of_key_tiles(B, S, H, mode):
     (12, 200, 12, torch.bfloat16, 'gelu', 'philox', 'uniform'),
     (5, 100, 16, torch.float16, 'relu', 'philox', 'feature_major'),  # other orders and padded rows
     (4, 512, 16, torch.float16, 'relu', 'explicit', 'uniform'),
+    (8, 128, 4, torch.float16, 'relu', 'philox', 'uniform'),         # the last token count with two sweeps over the keys,
+    (8, 128, 4, torch.float16, 'gelu', 'philox', 'uniform'),
+    (1, 1025, 4, torch.float16, 'relu', 'philox', 'uniform'),        # and the first with one
 ])
 def test_default_path_against_the_oracle(B, S, H, dtype, activation, mode, layouts):
     enc, dlin1 = run_private_case(B, S, H, layouts=layouts, activation=activation, mask_mode=mode, seed=S, dtype=dtype,
@@ -128,15 +131,15 @@ def test_private_passes_with_projections_stored_unit_by_unit():
         assert err <= 8 * HALF[torch.float16], (name, err)
 
 
-@pytest.mark.parametrize('B', [1, 4])
-def test_row_maxima_that_rise_by_more_than_the_lag(B):
+@pytest.mark.parametrize('B,activation', [(1, 'relu'), (1, 'gelu'), (4, 'gelu')])
+def test_row_maxima_that_rise_by_more_than_the_lag(B, activation):
     """Scores that grow along the keys by far more than 2^8 per tile: every tile raises the reference maximum and
-    rescales what has been summed so far (keys scaled up with their position).  512 tokens take two sweeps over the keys,
-    2048 one."""
+    rescales what has been summed so far (keys scaled up with their position).  ReLU layers sweep the keys of 512 tokens
+    twice, the others once (with ReLU only outputs are compared: rounding decides about whole elements behind its step)."""
     dev, S, H = torch.device('cuda:0'), 512, 2
     E = 64 * H
-    enc = Encoder('', B, S, H, E, L.uniform_layouts(), torch.float16, 0., 0., 0., 0., activation='gelu').to(dev)
-    ref = Encoder('', B, S, H, E, L.uniform_layouts(), torch.float16, 0., 0., 0., 0., activation='gelu',
+    enc = Encoder('', B, S, H, E, L.uniform_layouts(), torch.float16, 0., 0., 0., 0., activation=activation).to(dev)
+    ref = Encoder('', B, S, H, E, L.uniform_layouts(), torch.float16, 0., 0., 0., 0., activation=activation,
                   keep_all_intermediates=True).to(dev)
     gen = torch.Generator(device=dev).manual_seed(1)
     with torch.no_grad():
@@ -152,7 +155,7 @@ def test_row_maxima_that_rise_by_more_than_the_lag(B):
         y = e(xi)
         y.backward(torch.ones_like(y) * torch.linspace(-1, 1, E, device=dev).half())
         outs.append([y.detach(), xi.grad] + [q.grad for q in e.params])
-    for a, b in zip(*outs):
+    for a, b in list(zip(*outs))[:1 if activation == 'relu' else None]:
         assert torch.isfinite(b).all()
         # the keeping pass rounds scores of up to ~100 to 16 bits before exponentiating: errors of 2^-5 in ALPHA
         assert ((a.double() - b.double()).norm() / a.double().norm()).item() <= 2.0 ** -5
