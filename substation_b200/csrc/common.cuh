@@ -405,6 +405,12 @@ __device__ __forceinline__ float rcp_unit(float x) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+__device__ __forceinline__ float clamp_unit(float x, float lo, float hi) {   // a NaN stays one
+  float y;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(x), "f"(lo));
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(y), "f"(hi));
+  return y;
+}
 __device__ __forceinline__ float gelu_exponent(float x) { return x * fmaf(x * x, -0.10294324f, -2.3022082f); }
 
 __device__ __forceinline__ float act_fwd(float x, int activation) {
@@ -414,13 +420,14 @@ __device__ __forceinline__ float act_fwd(float x, int activation) {
 
 __device__ __forceinline__ float act_bwd(float x, float dy, int activation) {
   if (activation == SB_ACT_RELU) return x > 0.f ? dy : 0.f;
-  // d/dx of x * s(x) with s = 1 / (1 + q), q = 2^t as in act_fwd: s + x * s * (1 - s) * 2u', and 1 - s = q * s.  Past
-  // t = 126 (x below -10) s is zero, and x stops at 16 in magnitude, where the derivative is 0 or 1 to the last bit: q, s and
-  // the polynomial stay finite over the whole range of bf16, so that no product of a huge and a tiny factor is left standing.
-  const float xb = fabsf(x) > 16.f ? copysignf(16.f, x) : x;   // (a NaN stays)
-  const float x2 = xb * xb, t = gelu_exponent(xb);
-  const float q = ex2_unit(fminf(t, 126.f));
-  const float s = t > 126.f ? 0.f : rcp_unit(1.f + q);
+  // d/dx of x * s(x) with s = 1 / (1 + q), q = 2^t as in act_fwd: s + x * s * (1 - s) * 2u', and 1 - s = q * s.  x stops at
+  // -10, where t is just below 126 and the derivative -3e-36, and at 16, where it is 1 to the last bit: q, s and the polynomial
+  // stay finite over the whole range of bf16, so that no product of a huge and a tiny factor is left standing.  Two
+  // instructions: selecting 0 beyond the bounds cost 7 us of a B=16, L=384 training step.
+  const float xb = clamp_unit(x, -10.f, 16.f);
+  const float x2 = xb * xb;
+  const float q = ex2_unit(gelu_exponent(xb));
+  const float s = rcp_unit(1.f + q);
   return s * fmaf(xb * fmaf(x2, 0.21406448f, 1.5957691f), q * s, 1.f) * dy;
 }
 

@@ -182,6 +182,9 @@ def test_gelu_over_every_value_of_the_storage_type(dtype):
                             (dlin1, s + c * s * r * 2 * (2 / torch.pi) ** 0.5 * (1 + 3 * 0.044715 * c * c), 24)):
         assert torch.isfinite(got).all()
         assert ((got.double() - want).abs() <= unit * want.abs() + lost * 2.0 ** -24 + 2.0 ** -25).all()
+    x[0, 0, :3] = torch.tensor([float('nan'), float('inf'), -float('inf')], dtype=dtype)
+    ops.backward_dropout_activation_bias(torch.ones_like(x), mask, x, dlin1, bias.clone(), activation='gelu')
+    assert torch.isnan(dlin1[0, 0, 0]) and dlin1[0, 0, 1] == 1 and dlin1[0, 0, 2].double().abs() < 1e-30
 
 
 @pytest.mark.parametrize('B,J,F,lay', [(4, 64, 1024, 'BJI'), (2, 9, 200, 'BJI'), (2, 16, 128, 'IBJ'),
