@@ -462,7 +462,7 @@ class Encoder(torch.nn.Module):
     @staticmethod
     def _check_raw(device, **named):
         """The raw passes hand bare pointers to the library: every buffer must be dense and on the handle's
-        device.  Nothing is copied silently (a copy would also change the pointers the graph cache keys on)."""
+        device.  Nothing is copied silently: the caller's buffers are where results are expected."""
         for what, t in named.items():
             if isinstance(t, dict):
                 Encoder._check_raw(device, **{f'{what}[{k}]': v for k, v in t.items() if k != '__arena__'})
@@ -516,7 +516,8 @@ class Encoder(torch.nn.Module):
 
     def private_arena_bytes(self, device):
         """(forward, backward) arena bytes of passes whose intermediates nobody looks at (``forward_private``), or None
-        where such passes do not apply: ``enable_debug``, ``keep_all_intermediates``, ``profiling``, ``fuse=False``,
+        where such passes do not apply: ``enable_debug``, ``keep_all_intermediates``, ``profiling`` (``op_times`` lists the
+        operators of passes that store their results one by one), ``fuse=False``,
         a head size other than 64, samples of more than 2048 tokens."""
         with torch.cuda.device(device):
             plans = self._private_plans(torch.device('cuda', torch.cuda.current_device()))
@@ -695,7 +696,7 @@ class Encoder(torch.nn.Module):
 
     @property
     def encoder_func(self):
-        """The autograd function under the module (pytorch_module/encoder.py:78-139)."""
+        """The autograd function under the module (pytorch_module/encoder.py:78-139), as ``forward`` applies it."""
         return _BoundFunction(self)
 
     def forward(self, X):
@@ -704,5 +705,6 @@ class Encoder(torch.nn.Module):
             anchor = self.__dict__.get('_anchor')
             if anchor is None or anchor.device != X.device:
                 anchor = self._anchor = torch.zeros(1, device=X.device, requires_grad=True)
-            return self.encoder_func.apply(X, anchor, tuple(p.detach() for p in self.params))
-        return self.encoder_func.apply(X, None, *self.params)
+            return _EncoderFunction.apply(self, X, True, anchor, tuple(p.detach() for p in self.params))
+        keep = torch.is_grad_enabled() and (X.requires_grad or any(p.requires_grad for p in self.params))
+        return _EncoderFunction.apply(self, X, keep, None, *self.params)
