@@ -360,8 +360,8 @@ int sb_encoder_backward(sb_encoder* enc, void* stream, const void* dy, void* con
  * bit per score in `scratch` instead of the score tensors, and computes the scores again in the backward pass.  BETA,
  * ALPHA, ATTN_DROP, DATTN_DROP, DBETA and (philox) ATTN_DROP_MASK are neither read nor written, their table entries only
  * have to be non-null.  sb_encoder_private_bytes gives the two scratch sizes for a mask mode; both are 0 when these
- * passes do not apply: fusion off, dead stores on, head size other than 64, more than 2048 tokens per sample, or layouts the kernels do not read (the
- * passes themselves then return SB_ERR_UNSUPPORTED for the last two).  A backward pass takes the scratch of its forward
+ * passes do not apply: fusion off, dead stores on, head size other than 64, more than 2048 tokens per sample, or layouts the
+ * kernels do not read (the passes themselves then return SB_ERR_UNSUPPORTED for the last three).  A backward pass takes the scratch of its forward
  * pass, which must have run with keep != 0, and that pass's mask mode; scratch is 16-byte aligned.  Intermediates are kept in
  * orders of the library's choosing (same sizes, except that KKQQVV, WKKWQQWVV, GAMMA, DGAMMA and DKKQQVV hold rows of B * S
  * rounded up to a multiple of 8); x, y, dy, dx, parameters, their gradients and explicit masks keep the

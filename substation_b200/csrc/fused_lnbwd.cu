@@ -460,8 +460,9 @@ colsum_finish_kernel(const float* __restrict__ partial, int P, int F, void* o0, 
 // four consecutive tokens, one bulk copy per tensor and block).  Warps 0-27 consume, one warp per token: block i of
 // the CTA lives in stage i % NS and belongs to the warp set i % 7 (warps 4 * set .. 4 * set + 3, one token each), so
 // the seven blocks a CTA gets at 4096 tokens on 148 SMs are one round (sixteen warps took two: 18.3 against 16.5 us).
-// What only a backward pass reads (mask, DIFF, ISTD, LN) is not stored when its view is null.  Warp 28 produces.  A stage holds IN and RESID (4 x 2F bytes each) and, when the mask is an input, the mask rows
-// (4 x F bytes).  NV = 128-bit pieces per lane and row (F <= 256 * NV).
+// Warp 28 produces.  A stage holds IN and RESID (4 x 2F bytes each) and, when the mask is an input, the mask rows
+// (4 x F bytes).  NV = 128-bit pieces per lane and row (F <= 256 * NV).  What only a backward pass reads (mask, DIFF, ISTD,
+// LN) is not stored when its view is null.
 // ---------------------------------------------------------------------------------------------------------
 constexpr int kFwdWarps = 28;
 constexpr int kFwdThreads = (kFwdWarps + 1) * 32;
